@@ -550,6 +550,38 @@ static long long split_column(long long nz, long long cnt, int rows, bool shift,
   return n;
 }
 
+// Register chains (engine.cuh ChainCfg) stage nothing: no ring slots.
+static bool is_register_chain(const csd_kernel_desc& D) { return D.temporal > 1 && D.nslot == 0; }
+
+// Rows per item of a register chain (engine.cuh ChainCfg: one warp per item).
+// An item of r rows takes r + lead row times; a row's time grows slowly with
+// the blocks that share the SM, because the chain's latency is what they fill
+// (5-point heat, FP64, T = 5: 0.22, 0.27, 0.30, 0.37 us with 1 to 4 blocks of
+// four warps).  So the split that ends first trades the lead rows of many
+// short items against idle SMs under few long ones.  Measured per launch:
+// 1024^2 10.6 us with 12 rows per item, 14.2 with 8, 19.5 with 64; 4096^2
+// 68 us with 48 rows, 79 with 24, 83 with 128.
+static int chain_rows(long long columns, long long nz, long long lead, int warps_per_block,
+                      long long slots) {
+  const long long kSms = 148;
+  auto row_time = [&](long long blocks) { return 0.75 + 0.25 * (double)((blocks + kSms - 1) / kSms); };
+  long long best = nz;
+  double best_t = 0;
+  for (long long n = 1, tries = 0; n <= nz && tries < 128; n += 1 + n / 16, ++tries) {
+    const long long zc = (nz + n - 1) / n;
+    const long long blocks =
+        (columns * ((nz + zc - 1) / zc) + warps_per_block - 1) / warps_per_block;
+    double t = (double)(blocks / slots) * row_time(slots);
+    if (blocks % slots) t += row_time(blocks % slots);
+    t *= (double)(zc + lead);
+    if (best_t == 0 || t < best_t) {
+      best_t = t;
+      best = zc;
+    }
+  }
+  return (int)best;
+}
+
 int csd_plan_items(const csd_kernel_desc* D, long long slots, int zchunk_req, csd_grid* g) {
   if (!D || !g) return fail(CSD_EINVAL, "null argument");
   if (D->rows < 1 || g->tiles[0] < 1 || g->tiles[1] < 1 || g->interior[0] < 1)
@@ -562,6 +594,10 @@ int csd_plan_items(const csd_kernel_desc* D, long long slots, int zchunk_req, cs
   const int rows = D->rows;
   const long long columns = (long long)g->tiles[0] * g->tiles[1];
   int zchunk = zchunk_req > 0 ? zchunk_req : D->zchunk;
+  if (is_register_chain(*D) && zchunk_req <= 0)
+    // lead: 2 T RZ input rows, T steps of skew, and about four rows' time
+    // before the first input arrives
+    zchunk = chain_rows(columns, nz, 2ll * D->rz + D->temporal + 4, D->threads / 32, slots);
   const bool one_wave = zchunk_req <= 0 && D->zchunk == 0;
   if (zchunk <= 0) {
     // -W: W items per resident block (issue-bound bodies balance better)
@@ -631,6 +667,13 @@ int csd_grid_item_place(const csd_grid* g, int item, int* tx, int* ty, int* z0, 
   if (item < 0 || item >= g->items) return fail(CSD_EINVAL, "item %d out of [0, %d)", item, g->items);
   csd_item_place(g, item, tx, ty, z0, nrows);
   return CSD_OK;
+}
+
+// Blocks that hold `items` work items: one item per block, or per warp of a
+// register chain.
+static int item_blocks(const csd_kernel_desc& D, int items) {
+  const int per = is_register_chain(D) ? D.threads / 32 : 1;
+  return (int)(((long long)items + per - 1) / per);
 }
 
 static int build_grid(csd_kernel* k, const csd_field* in, int n_in, const csd_field* out,
@@ -764,7 +807,7 @@ static int build_grid(csd_kernel* k, const csd_field* in, int n_in, const csd_fi
                                    0);
       if (r) return cu_fail(r, "cuTensorMapEncodeTiled(brick rows)");
     }
-  } else if (loader == CSD_LOADER_TMA) {
+  } else if (loader == CSD_LOADER_TMA && !is_register_chain(D)) {
     Driver& d = drv();
     for (int i = 0; i < n_in; ++i) {
       unsigned long long gdim[3] = {(unsigned long long)g->dims[2], (unsigned long long)g->dims[1],
@@ -826,7 +869,8 @@ int csd_launch(csd_kernel* k, const csd_field* in, int n_in, const csd_field* ou
   p.timeout_ns = o.timeout_ns ? o.timeout_ns : 2000000000ull;
   p.withhold = o.withhold_chunk > 0 ? o.withhold_chunk : 0;
   int grid = o.grid > 0 ? o.grid : k->blocks_per_sm[loader] * st->sms;
-  if (grid > p.g.items) grid = p.g.items;
+  const int blocks = item_blocks(k->desc, p.g.items);
+  if (grid > blocks) grid = blocks;
   if (grid < 1) return CSD_OK;  // nothing to do
   void* args[] = {&p};
   CUresult r = drv().cuLaunchKernel(k->fn[loader], (unsigned)grid, 1, 1, (unsigned)k->desc.threads,
@@ -880,7 +924,8 @@ int csd_launch_batch(csd_kernel* k, const csd_grid* grids, const int* item_start
   p.withhold = (opts && opts->withhold_chunk > 0) ? opts->withhold_chunk : 0;
   const int loader = (opts && opts->loader == CSD_LOADER_LDG) ? CSD_LOADER_LDG : CSD_LOADER_TMA;
   int grid = (opts && opts->grid > 0) ? opts->grid : k->blocks_per_sm[loader] * st->sms;
-  if (grid > total_items) grid = total_items;
+  const int blocks = item_blocks(k->desc, total_items);
+  if (grid > blocks) grid = blocks;
   void* args[] = {&p};
   CUresult r = drv().cuLaunchKernel(k->fn[loader], (unsigned)grid, 1, 1,
                                     (unsigned)k->desc.threads, 1, 1, (unsigned)k->desc.smem_bytes,

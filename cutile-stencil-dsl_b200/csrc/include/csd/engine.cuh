@@ -643,6 +643,275 @@ __device__ __forceinline__ int batch_grid_of(const csd_params& p, int item, int&
 }
 
 // ---------------------------------------------------------------------------
+// Register chains: 1-D and 2-D temporal blocking without shared memory
+// ---------------------------------------------------------------------------
+// A work item is one warp's: a strip of TX columns, the warp's 32 x VEC
+// points (VEC neighbouring columns per lane) covering the strip and the
+// columns the T steps consume on either side.  The warp walks the rows of its
+// item with the 2 RZ + 1 newest rows of each of the T fields in registers and
+// reads X neighbours from the neighbouring lanes by shuffles: no barrier and
+// no shared memory stand between the stages.  Stage s reads only rows of
+// field s - 1 that earlier steps finished, so the T stages of a step are
+// independent and hide each other's latency; running them from the last to
+// the first lets the new row of a field take the place of the row that the
+// stage above has just read for the last time.  Input rows arrive DEPTH steps
+// ahead by cp.async into a ring of the lane's own 16-byte groups (each lane
+// reads back only what it copied, so the copies need no barrier either; loads
+// into registers that far ahead measured slower: a step then waits for the
+// youngest of them).  What bounds it is
+// instruction issue: the body's own arithmetic, the shuffles, and the strip's
+// T RX columns and the item's 2 T RZ rows that are computed twice.
+template <typename T_, int NIN_, int NOUT_, int RZ_, int RX_, int NT_, int TEMPORAL_, int LOADER_,
+          int VEC_>
+struct ChainCfg {
+  typedef T_ T;
+  static constexpr int NIN = NIN_, NOUT = NOUT_;
+  static constexpr int RZ = RZ_, RY = 0, RX = RX_;   // radius of ONE step
+  static constexpr int NT = NT_, TEMPORAL = TEMPORAL_, LOADER = LOADER_, VEC = VEC_;
+  static constexpr int ALIGN = 16 / (int)sizeof(T);
+  static constexpr int W = 2 * RZ + 1;               // rows of a field's register window
+  static constexpr int PADL = cdiv(TEMPORAL * RX, VEC) * VEC;
+  static constexpr int TX = (32 * VEC - PADL - TEMPORAL * RX) / VEC * VEC;   // columns stored
+  // what the kernel descriptor names; NSLOT = 0 tells the host that items are
+  // per warp and stage nothing in shared memory
+  static constexpr int ROWS = 1, TY = 1, RPY = 1, STAGES = 0, NSLOT = 0, HC = RZ;
+  static constexpr int BOXW = 32 * VEC, BOXH = 1, BC = CSD_BC_NONE, BRICK_SHIFT = 0;
+  static constexpr int DEPTH = RZ > 0 ? 8 : 0;       // input rows in flight
+  static constexpr int ROW_BYTES = NT * VEC * (int)sizeof(T);   // one row of every lane
+  static constexpr int SMEM_BYTES = DEPTH * NIN * ROW_BYTES;
+  static_assert(VEC % ALIGN == 0, "a lane owns whole 16-byte vectors");
+  static_assert(TX > 0, "the chain consumes the whole strip");
+  static_assert(NIN == NOUT, "a temporal chain feeds output field f into input field f");
+};
+
+// The rows a stage reads, for the body functor: window row DZ of a field,
+// with the columns past the lane's own points taken from its neighbours.
+template <class C>
+struct ChainView {
+  typedef typename C::T T;
+  const T (*win)[C::W][C::VEC];   // [field][row slot][point], registers
+  int oldest;                     // slot of row -RZ (constant once unrolled)
+  const double* scal;
+  const double* dyn;
+
+  __device__ __forceinline__ double scalar(int k) const { return scal[k]; }
+  __device__ __forceinline__ double dynamic(int k) const { return dyn[k]; }
+
+  template <int F, int DZ, int DY, int LO, int HI>
+  __device__ __forceinline__ Strip<T, LO, HI, C::VEC> strip(int, int, int) const {
+    const T* row = win[F][(oldest + C::RZ + DZ) % C::W];
+    Strip<T, LO, HI, C::VEC> s;
+#pragma unroll
+    for (int i = 0; i < C::VEC + HI - LO; ++i) {
+      const int q = fdiv(LO + i, C::VEC);      // neighbouring lane that owns the column
+      const T v = row[LO + i - q * C::VEC];
+      s.v[i] = q == 0 ? v
+                      : (q < 0 ? __shfl_up_sync(0xffffffffu, v, -q)
+                               : __shfl_down_sync(0xffffffffu, v, q));
+    }
+    return s;
+  }
+};
+
+// One item.  MASKED: some intermediate point or input cell of the item lies
+// outside the interior (such points are zero, as the zero-halo buffers of
+// separate launches hold; cells outside the array are never read).
+template <class C, class Body, bool MASKED>
+__device__ __forceinline__ void chain_item(const csd_grid& g, int gx0, int z0, int nrows) {
+  typedef typename C::T T;
+  constexpr int T_ = C::TEMPORAL, W = C::W, V = C::VEC, RZ = C::RZ;
+  const int lane = threadIdx.x & 31;
+  const int nz = g.interior[0];
+  const int hx = g.halo[2], xend = g.halo[2] + g.interior[2];
+  const int NZ = (int)g.dims[0], NX = (int)g.dims[2];
+  const long long pitch = g.pitch_z;
+  const bool xall = !MASKED || (gx0 >= 0 && gx0 + V <= NX);        // all points in the array
+  const bool xin = gx0 >= hx && gx0 + V <= xend;                   // ... in the interior
+  const bool owner = lane >= C::PADL / V && lane < (C::PADL + C::TX) / V;
+  const bool vec_store = g.vec_store != 0;
+  bool in[V];
+#pragma unroll
+  for (int e = 0; e < V; ++e) in[e] = gx0 + e >= hx && gx0 + e < xend;
+  const int n = nrows + 2 * T_ * RZ;               // input rows of the item
+  const int zin = g.halo[0] + z0 - T_ * RZ;        // array row of input row 0
+  const T* src[C::NIN];
+  T* dst[C::NOUT];
+#pragma unroll
+  for (int f = 0; f < C::NIN; ++f)
+    src[f] = reinterpret_cast<const T*>(g.in[f]) + (long long)zin * pitch + gx0;
+#pragma unroll
+  for (int f = 0; f < C::NOUT; ++f)
+    dst[f] = reinterpret_cast<T*>(g.out[f]) + (long long)(g.halo[0] + z0) * pitch + gx0;
+
+  // stores one row of the item; dst moves on to the next
+  auto store_row = [&](const OutPack<T, C::NOUT, V>& o) {
+#pragma unroll
+    for (int f = 0; f < C::NOUT; ++f) {
+      if (owner) {
+        if (vec_store && (!MASKED || xin)) {
+          store_unit<V>(dst[f], o.v[f]);
+        } else {
+#pragma unroll
+          for (int e = 0; e < V; ++e)
+            if (!MASKED || in[e]) dst[f][e] = o.v[f][e];
+        }
+      }
+      dst[f] += pitch;
+    }
+  };
+  // an intermediate value of interior row zr
+  auto masked = [&](T v, int e, int zr) {
+    return !MASKED || (in[e] && (unsigned)zr < (unsigned)nz) ? v : T(0);
+  };
+
+  if constexpr (RZ == 0) {
+    // no rows to wait for: each row takes its T steps at once
+#pragma unroll 1
+    for (int j = 0; j < n; ++j) {
+      T win[C::NIN][1][V];
+      const bool row = !MASKED || (zin + j >= 0 && zin + j < NZ);
+#pragma unroll
+      for (int f = 0; f < C::NIN; ++f) {
+        if (C::LOADER == CSD_LOADER_TMA && row && xall) {
+          typedef typename VecOf<T>::type Q;
+#pragma unroll
+          for (int e = 0; e < V; e += C::ALIGN)
+            *reinterpret_cast<Q*>(&win[f][0][e]) = __ldg(reinterpret_cast<const Q*>(src[f] + e));
+        } else {
+#pragma unroll
+          for (int e = 0; e < V; ++e) {
+            win[f][0][e] = T(0);
+            if (row && (!MASKED || (gx0 + e >= 0 && gx0 + e < NX)))
+              win[f][0][e] = __ldg(src[f] + e);
+          }
+        }
+        src[f] += pitch;
+      }
+#pragma unroll
+      for (int s = 1; s <= T_; ++s) {
+        OutPack<T, C::NOUT, V> o;
+        const ChainView<C> view{win, 0, g.scalars, g.dyn};
+        Body::template compute<C>(view, 0, 0, 0, o);
+        if (s == T_) {
+          store_row(o);
+        } else {
+#pragma unroll
+          for (int f = 0; f < C::NOUT; ++f)
+#pragma unroll
+            for (int e = 0; e < V; ++e) win[f][0][e] = masked(o.v[f][e], e, z0 + j);
+        }
+      }
+    }
+  } else {
+    constexpr int D = C::DEPTH;
+    extern __shared__ __align__(128) unsigned char smem_dyn[];
+    T* own = reinterpret_cast<T*>(smem_dyn) + threadIdx.x * V;   // + slot and field rows
+    constexpr int FROW = C::ROW_BYTES / (int)sizeof(T);
+    const unsigned own_addr = ptx::smem_addr(own);
+    // request input row j (the next one; src moves on to the row after it)
+    // (selects, not branches: a step stays one block of independent work)
+    auto request_row = [&](int j) {
+      const bool row = j < n && (!MASKED || (zin + j >= 0 && zin + j < NZ));
+      const unsigned to = own_addr + (unsigned)((j % D) * C::NIN) * C::ROW_BYTES;
+#pragma unroll
+      for (int f = 0; f < C::NIN; ++f) {
+        const T* base = reinterpret_cast<const T*>(g.in[f]);
+        constexpr int STEP = C::LOADER == CSD_LOADER_TMA ? C::ALIGN : 1;   // points per copy
+#pragma unroll
+        for (int e = 0; e < V; e += STEP) {
+          int have = STEP;   // points of the copy inside the array
+          if (MASKED) have = gx0 + e < 0 ? 0 : min(max(NX - (gx0 + e), 0), STEP);
+          if (!row) have = 0;
+          const T* from = have > 0 ? src[f] + e : base;
+          const unsigned at = to + f * C::ROW_BYTES + e * (int)sizeof(T);
+          if constexpr (STEP > 1)
+            ptx::cp_async_16_partial(at, from, have * (int)sizeof(T));
+          else
+            ptx::cp_async_zfill<sizeof(T)>(at, from, have > 0);
+        }
+        src[f] += pitch;
+      }
+      ptx::cp_async_commit();   // one group per row, empty past the last
+    };
+    T win[T_][C::NIN][W][V];   // the W newest rows of the input and of every intermediate field
+#pragma unroll
+    for (int s = 0; s < T_; ++s)
+#pragma unroll
+      for (int f = 0; f < C::NIN; ++f)
+#pragma unroll
+        for (int u = 0; u < W; ++u)
+#pragma unroll
+          for (int e = 0; e < V; ++e) win[s][f][u][e] = T(0);
+#pragma unroll 1
+    for (int j = 0; j < D - 1; ++j) request_row(j);
+    // Step j takes in input row j; stage s computes row j - s - s RZ of its
+    // field, from rows that are there from step s W on.
+#pragma unroll 1
+    for (int j0 = 0; j0 < n + T_; j0 += W) {
+#pragma unroll
+      for (int u = 0; u < W; ++u) {
+        const int j = j0 + u;
+#pragma unroll
+        for (int s = T_; s >= 1; --s) {
+          OutPack<T, C::NOUT, V> o;
+          const ChainView<C> view{win[s - 1], u, g.scalars, g.dyn};
+          Body::template compute<C>(view, 0, 0, 0, o);
+          if (s == T_) {
+            if (j0 >= T_ * W && j < n + T_) store_row(o);
+          } else {
+            const int zr = z0 - T_ * RZ + j - s - s * RZ;
+#pragma unroll
+            for (int f = 0; f < C::NOUT; ++f)
+#pragma unroll
+              for (int e = 0; e < V; ++e)
+                win[s < T_ ? s : 0][f][u][e] = masked(o.v[f][e], e, zr);
+          }
+        }
+        // row j - 1, whose slot the next request takes, was read by stage 1 above
+        request_row(j + D - 1);
+        ptx::cp_async_wait<D - 1>();
+        typedef typename VecOf<T>::type Q;
+#pragma unroll
+        for (int f = 0; f < C::NIN; ++f)
+#pragma unroll
+          for (int e = 0; e < V; e += C::ALIGN)
+            *reinterpret_cast<Q*>(&win[0][f][u][e]) =
+                *reinterpret_cast<const Q*>(own + ((j % D) * C::NIN + f) * FROW + e);
+      }
+    }
+    ptx::cp_async_wait<0>();   // the ring is free for the warp's next item
+  }
+}
+
+template <class C, class Body, bool BATCHED>
+__device__ __forceinline__ void chain_items(const csd_params& p) {
+  constexpr int T_ = C::TEMPORAL, NW = C::NT / 32;
+  const int total = BATCHED ? p.total_items : p.g.items;
+  for (int gitem = blockIdx.x * NW + (threadIdx.x >> 5); gitem < total; gitem += gridDim.x * NW) {
+    int item = gitem;
+    const csd_grid& g = BATCHED ? p.grids[batch_grid_of(p, gitem, item)] : p.g;
+    int tx, ty, z0, nrows;
+    csd_item_place(&g, item, &tx, &ty, &z0, &nrows);
+    const int x0 = g.xbase + tx * C::TX - C::PADL;   // array column of the warp's first point
+    const bool inside = x0 >= g.halo[2] && x0 + 32 * C::VEC <= g.halo[2] + g.interior[2] &&
+                        z0 - T_ * C::RZ >= 0 && z0 + nrows + T_ * C::RZ <= g.interior[0];
+    const int gx0 = x0 + (int)(threadIdx.x & 31) * C::VEC;
+    if (inside)
+      chain_item<C, Body, false>(g, gx0, z0, nrows);
+    else
+      chain_item<C, Body, true>(g, gx0, z0, nrows);
+  }
+}
+
+template <class C, class Body>
+__device__ __forceinline__ void register_chain(const csd_params& p) {
+  if (p.grids == nullptr)
+    chain_items<C, Body, false>(p);
+  else
+    chain_items<C, Body, true>(p);
+}
+
+// ---------------------------------------------------------------------------
 // The engine
 // ---------------------------------------------------------------------------
 template <class C, class Body, bool BATCHED>

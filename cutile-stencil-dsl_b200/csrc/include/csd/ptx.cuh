@@ -109,6 +109,14 @@ __device__ __forceinline__ void cp_async_16_partial(unsigned dst, const void* sr
                : "memory");
 }
 
+// Close this thread's current group of cp.async copies; wait until at most N
+// of its most recent groups are still in flight.
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
 // Arrive on `bar` once all of this thread's prior cp.async copies land.
 __device__ __forceinline__ void cp_async_arrive(unsigned bar) {
   asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");

@@ -217,8 +217,8 @@ def emit_body(kernel: KernelOp) -> str:
     unroll = 4 if (len(gkeys) <= 8 and rpy == 1 and body_lines <= 48) else 0
     out = [f"struct Body_{name} {{",
            f"  static constexpr int UNROLL = {unroll};",
-           "  template <class C>",
-           "  __device__ __forceinline__ static void compute(const csd::TileView<C>& t, int r, int y,",
+           "  template <class C, class View>",
+           "  __device__ __forceinline__ static void compute(const View& t, int r, int y,",
            "                                                 int x, csd::OutPack<typename C::T, "
            "C::NOUT, C::VEC * C::RPY>& o) {",
            f"    static_assert(C::VEC == {vec} && C::RPY == {rpy}, "
@@ -316,6 +316,9 @@ def emit_body(kernel: KernelOp) -> str:
     return "\n".join(out)
 
 
+CHAIN_THREADS = 128   # four independent warps per block of a register chain
+
+
 def _internal_radius(ndim: int, radius) -> tuple[int, int, int]:
     r = list(radius)
     if ndim == 3:
@@ -361,7 +364,10 @@ def engine_params(kernel: KernelOp) -> dict:
         "REDUCE": kernel.reduce_max.data if kernel.reduce_max is not None else 0,
         "BRICK": _brick_code(kernel, ndim),
         "RPY": int(hints.get("rpy", 1)),
-        "VEC": int(hints.get("vec", 4 if dtype in ("float32", "fp32") else 2)),
+        # points per lane of a register chain (0: the ring engine)
+        "CHAIN": int(hints.get("register_chain", 0)),
+        "VEC": int(hints.get("register_chain", 0)
+                   or hints.get("vec", 4 if dtype in ("float32", "fp32") else 2)),
     }
 
 
@@ -422,13 +428,18 @@ def emit_cuda(module: ModuleOp, preamble: bool = True) -> str:
         for suffix, loader in (("tma", "CSD_LOADER_TMA"), ("ldg", "CSD_LOADER_LDG")):
             if p["BRICK"] and not brick_tma:
                 loader = "CSD_LOADER_LDG"   # bricked fields the TMA boxes cannot stage
+            entry, nt, minb = "stream_engine", p["NT"], p["MINB"]
             cfg = (f"csd::Cfg<{p['T']}, {p['NIN']}, {p['NOUT']}, {p['RZ']}, {p['RY']}, {p['RX']}, "
                    f"{p['ROWS']}, {p['TY']}, {p['TX']}, {p['NT']}, {p['STAGES']}, {p['TEMPORAL']}, "
                    f"{loader}, {p['BC']}, {p['REDUCE']}, {p['BRICK']}, {p['RPY']}, {p['VEC']}>")
+            if p["CHAIN"]:
+                entry, nt, minb = "register_chain", CHAIN_THREADS, 1
+                cfg = (f"csd::ChainCfg<{p['T']}, {p['NIN']}, {p['NOUT']}, {p['RZ']}, {p['RX']}, "
+                       f"{nt}, {p['TEMPORAL']}, {loader}, {p['VEC']}>")
             parts.append(f"typedef {cfg} Cfg_{name}_{suffix};")
-            parts.append(f'extern "C" __global__ void __launch_bounds__({p["NT"]}, {p["MINB"]})')
+            parts.append(f'extern "C" __global__ void __launch_bounds__({nt}, {minb})')
             parts.append(f"{name}_{suffix}(const __grid_constant__ csd_params p) {{")
-            parts.append(f"  csd::stream_engine<Cfg_{name}_{suffix}, Body_{name}>(p);")
+            parts.append(f"  csd::{entry}<Cfg_{name}_{suffix}, Body_{name}>(p);")
             parts.append("}")
         c = f"Cfg_{name}_tma"
         parts.append(f'extern "C" __device__ const csd_kernel_desc {name}_desc = {{')

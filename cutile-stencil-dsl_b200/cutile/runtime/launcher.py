@@ -490,6 +490,36 @@ def chain_tile_2d(dtype_bytes: int, T: int) -> dict:
     return dict(rows=4, tile_x=128, threads=256)
 
 
+def register_chain_points(radius, dtype_bytes: int, num_inputs: int, T: int,
+                          body_ops: int) -> int:
+    """Points per lane of the register chain (engine.cuh ``ChainCfg``) for a
+    chain of T steps, or 0 where the shared-memory rings keep it.
+
+    1-D and 2-D chains whose windows fit the registers take it.  Measured on
+    B200 per launch, rings -> registers: heat 1024^2 FP64 T=5 103 -> 10.9 us,
+    4096^2 323 -> 68; FP32 T=8 194 -> 13.2 and 472 -> 62; Kahan T=4 80 -> 12.6
+    and 275 -> 73; radius 2 FP64 T=4 80 -> 25 and 315 -> 170; heat1d 2^22 T=8
+    FP64 123 -> 18, FP32 68 -> 10.  The one loss seen is a radius-2 FP32 chain
+    of three or four steps on a grid too small to fill the chip (200 x 300:
+    8.5 -> 9.9 and 12.2 -> 16.0 us; 1024^2: 28 -> 15 and 51 -> 28)."""
+    ndim = len(radius)
+    if ndim > 2:
+        return 0
+    rz, rx = (radius[0] if ndim == 2 else 0), radius[-1]
+    # one 16-byte vector per lane; two in 1-D, where no rows are kept (FP32
+    # 2^22: 14.8 us with one, 10.1 with two, 10.2 with four)
+    vec = 16 // dtype_bytes * (2 if ndim == 1 else 1)
+    # registers of the T windows (192: two blocks per SM still beat the rings,
+    # Kahan T=8 1094 -> 139 us at 4096^2; past that they spill), and the
+    # unrolled code (2 rz + 1 copies of every stage's body)
+    window = T * num_inputs * (2 * rz + 1) * vec * dtype_bytes // 4
+    if window > 192 or T * (2 * rz + 1) * body_ops > 3000:
+        return 0
+    # the strip's stored columns: at least half of the 32 lanes' points
+    pad = -(-T * rx // vec) * vec
+    return vec if 2 * (32 * vec - pad - T * rx) >= 32 * vec else 0
+
+
 def _rpy_keeps_registers(stencil_fn, plan, stencil_halo, halo_widths, dtype, dtype_bytes,
                          num_inputs, T, body_ops, kahan) -> bool:
     """Whether the rows-per-thread default compiles without spills for this
@@ -637,6 +667,14 @@ def compile(stencil_fn, domain: tuple[int, ...] | None = None, hw=None,
     hints = plan.hints()
     if occupancy is not None:
         hints["occupancy"] = occupancy
+    if T > 1 and layout != "bricked":
+        if kernel_hints and "register_chain" in kernel_hints:
+            hints["register_chain"] = int(kernel_hints["register_chain"])
+        elif tile_sizes is None and not kernel_hints and occupancy is None:
+            points = register_chain_points(stencil_halo, dtype_bytes, num_inputs, T,
+                                           analysis.get("body_ops", 0))
+            if points:
+                hints["register_chain"] = points
 
     boundary_spec = None
     if getattr(stencil_fn, "_boundary", None) is not None:

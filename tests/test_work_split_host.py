@@ -103,3 +103,15 @@ def test_chains_default_to_eight_waves():
     p1 = fit_plan(EnginePlan(3, rows=1, tile_y=4, tile_x=128, vec=2, threads=128, stages=1,
                              zchunk=0), (1, 1, 1), 8, 1)
     assert p1.waves == 1
+
+
+@pytest.mark.parametrize("tiles_x,nz", [(1, 1), (1, 7), (20, 1024), (79, 4096), (3, 100000)])
+def test_register_chain_items_cover_every_row_once(tiles_x, nz):
+    """Items of a register chain (no ring slots, one warp each): every row of
+    every strip exactly once."""
+    from cutile.runtime import native
+
+    desc = {"rows": 1, "threads": 128, "nslot": 0, "temporal": 5, "rz": 5, "zchunk": -8}
+    split, items = native.plan_items(desc, tiles_x, 1, nz, 592)
+    seen = sorted((tx, z) for tx, ty, z0, n in items for z in range(z0, z0 + n))
+    assert seen == [(tx, z) for tx in range(tiles_x) for z in range(nz)]
