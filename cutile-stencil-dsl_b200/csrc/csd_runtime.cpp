@@ -345,6 +345,10 @@ struct csd_kernel {
   CUfunction fn[2] = {nullptr, nullptr};  // [CSD_LOADER_TMA], [CSD_LOADER_LDG]
   csd_kernel_desc desc;
   int blocks_per_sm[2] = {0, 0};
+  // the kernel's direct form (engine.cuh DirectCfg), when its module has one
+  CUfunction direct = nullptr;
+  csd_kernel_desc direct_desc;
+  int direct_blocks_per_sm = 0;
   std::string name;
 };
 
@@ -477,6 +481,16 @@ int csd_kernel_get(csd_module* m, const char* name, csd_kernel** out) {
     }
     if (k->blocks_per_sm[l] < 1) k->blocks_per_sm[l] = 1;
   }
+  CUfunction direct = nullptr;
+  if (d.cuModuleGetFunction(&direct, m->mod, (n + "_direct").c_str()) == 0 &&
+      d.cuModuleGetGlobal(&dp, &sz, m->mod, (n + "_direct_desc").c_str()) == 0 &&
+      sz == sizeof(csd_kernel_desc) &&
+      d.cuMemcpyDtoH(&k->direct_desc, dp, sizeof(csd_kernel_desc)) == 0 &&
+      k->direct_desc.magic == CSD_DESC_MAGIC &&
+      d.cuOccupancyMaxActiveBlocksPerMultiprocessor(&k->direct_blocks_per_sm, direct,
+                                                    k->direct_desc.threads, 0) == 0 &&
+      k->direct_blocks_per_sm > 0)
+    k->direct = direct;
   *out = k;
   return CSD_OK;
 }
@@ -550,8 +564,16 @@ static long long split_column(long long nz, long long cnt, int rows, bool shift,
   return n;
 }
 
-// Register chains (engine.cuh ChainCfg) stage nothing: no ring slots.
+// Register chains and direct kernels (engine.cuh ChainCfg, DirectCfg) stage
+// nothing: they have no ring slots.
 static bool is_register_chain(const csd_kernel_desc& D) { return D.temporal > 1 && D.nslot == 0; }
+static bool is_direct(const csd_kernel_desc& D) {
+  return D.temporal == 1 && D.nslot == 0 && D.threads > 0;
+}
+// An item of theirs is a warp's (a direct 3-D kernel's: the block's).
+static int warps_per_item(const csd_kernel_desc& D) {
+  return is_register_chain(D) || (is_direct(D) && D.tile_y == 1) ? 1 : D.threads / 32;
+}
 
 // Rows per item of a register chain (engine.cuh ChainCfg: one warp per item).
 // An item of r rows takes r + lead row times; a row's time grows slowly with
@@ -598,6 +620,10 @@ int csd_plan_items(const csd_kernel_desc* D, long long slots, int zchunk_req, cs
     // lead: 2 T RZ input rows, T steps of skew, and about four rows' time
     // before the first input arrives
     zchunk = chain_rows(columns, nz, 2ll * D->rz + D->temporal + 4, D->threads / 32, slots);
+  // a direct kernel's lead is the 2 RZ rows it reads again; the split that suits
+  // a chain measured within 5 % of the best of 8 to 301 rows here too
+  if (is_direct(*D) && zchunk_req <= 0)
+    zchunk = chain_rows(columns, nz, 2ll * D->rz + 4, D->threads / 32 / warps_per_item(*D), slots);
   const bool one_wave = zchunk_req <= 0 && D->zchunk == 0;
   if (zchunk <= 0) {
     // -W: W items per resident block (issue-bound bodies balance better)
@@ -669,17 +695,25 @@ int csd_grid_item_place(const csd_grid* g, int item, int* tx, int* ty, int* z0, 
   return CSD_OK;
 }
 
+// csd_launch's own choice of copy path, and the path it may add to
+// CSD_LOADER_TMA and CSD_LOADER_LDG.
+static const int kLoaderAny = -2, kLoaderDirect = 2;
+
+static int resident_blocks(const csd_kernel* k, int loader) {
+  return loader == kLoaderDirect ? k->direct_blocks_per_sm : k->blocks_per_sm[loader];
+}
+
 // Blocks that hold `items` work items: one item per block, or per warp of a
 // register chain.
 static int item_blocks(const csd_kernel_desc& D, int items) {
-  const int per = is_register_chain(D) ? D.threads / 32 : 1;
+  const int per = D.nslot == 0 && D.threads > 0 ? D.threads / 32 / warps_per_item(D) : 1;
   return (int)(((long long)items + per - 1) / per);
 }
 
 static int build_grid(csd_kernel* k, const csd_field* in, int n_in, const csd_field* out,
                       int n_out, const csd_launch_opts& o, DeviceState* st, int loader_req,
                       csd_grid* g, int* loader_out) {
-  const csd_kernel_desc& D = k->desc;
+  csd_kernel_desc D = k->desc;
   if (!in || (!out && n_out > 0)) return fail(CSD_EINVAL, "null field array");
   if (D.reduce_max && !o.red)
     return fail(CSD_EINVAL, "kernel %s max-reduces: opts.red must point to a device double",
@@ -753,7 +787,12 @@ static int build_grid(csd_kernel* k, const csd_field* in, int n_in, const csd_fi
                                    : D.brick_tma != 0;
   for (int i = 0; i < n_in; ++i) tma_ok = tma_ok && (reinterpret_cast<uintptr_t>(in[i].ptr) % 16 == 0);
   int loader = loader_req;
-  if (loader < 0 || loader > 1) loader = tma_ok ? CSD_LOADER_TMA : CSD_LOADER_LDG;
+  if (loader == kLoaderAny) {   // csd_launch: the direct kernel takes unaligned rows
+    loader = tma_ok ? CSD_LOADER_TMA : k->direct ? kLoaderDirect : CSD_LOADER_LDG;
+    if (loader == kLoaderDirect) D = k->direct_desc;
+  } else if (loader < 0 || loader > 1) {
+    loader = tma_ok ? CSD_LOADER_TMA : CSD_LOADER_LDG;
+  }
   if (loader == CSD_LOADER_TMA && !tma_ok)
     return fail(CSD_EALIGN, "TMA path needs 16-byte aligned fields and row pitch");
   const bool brick_tma = D.brick_shift > 0 && loader == CSD_LOADER_TMA;
@@ -763,11 +802,13 @@ static int build_grid(csd_kernel* k, const csd_field* in, int n_in, const csd_fi
   // outside the interior are computed but never stored.  (The tile height
   // divides the brick or is a multiple of it, so every brick row a tile
   // covers starts a box.)
+  // Direct kernels read any column, so their tiles start at the interior.
   g->xbase = brick_tma ? (int)((g->halo[2] / B) * B) : (g->halo[2] / D.align) * D.align;
+  if (loader == kLoaderDirect) g->xbase = g->halo[2];
   g->ybase = brick_tma ? (g->halo[1] / D.tile_y) * D.tile_y : g->halo[1];
   g->tiles[0] = (g->halo[2] + g->interior[2] - g->xbase + D.tile_x - 1) / D.tile_x;
   g->tiles[1] = (g->halo[1] + g->interior[1] - g->ybase + D.tile_y - 1) / D.tile_y;
-  const long long slots = o.grid > 0 ? o.grid : (long long)k->blocks_per_sm[loader] * st->sms;
+  const long long slots = o.grid > 0 ? o.grid : (long long)resident_blocks(k, loader) * st->sms;
   int rc = csd_plan_items(&D, slots, o.zchunk, g);
   if (rc) return rc;
   g->bc_value = o.bc_value;
@@ -863,18 +904,22 @@ int csd_launch(csd_kernel* k, const csd_field* in, int n_in, const csd_field* ou
   csd_params p;
   memset(&p, 0, sizeof(p));
   int loader = 0;
-  rc = build_grid(k, in, n_in, out, n_out, o, st, o.loader, &p.g, &loader);
+  // a withheld input chunk needs a kernel that stages chunks
+  const bool any = (o.loader < 0 || o.loader > 1) && o.withhold_chunk <= 0;
+  rc = build_grid(k, in, n_in, out, n_out, o, st, any ? kLoaderAny : o.loader, &p.g, &loader);
   if (rc) return rc;
+  const csd_kernel_desc& D = loader == kLoaderDirect ? k->direct_desc : k->desc;
   p.err = reinterpret_cast<int*>(st->err);
   p.timeout_ns = o.timeout_ns ? o.timeout_ns : 2000000000ull;
   p.withhold = o.withhold_chunk > 0 ? o.withhold_chunk : 0;
-  int grid = o.grid > 0 ? o.grid : k->blocks_per_sm[loader] * st->sms;
-  const int blocks = item_blocks(k->desc, p.g.items);
+  int grid = o.grid > 0 ? o.grid : resident_blocks(k, loader) * st->sms;
+  const int blocks = item_blocks(D, p.g.items);
   if (grid > blocks) grid = blocks;
   if (grid < 1) return CSD_OK;  // nothing to do
   void* args[] = {&p};
-  CUresult r = drv().cuLaunchKernel(k->fn[loader], (unsigned)grid, 1, 1, (unsigned)k->desc.threads,
-                                    1, 1, (unsigned)k->desc.smem_bytes,
+  CUresult r = drv().cuLaunchKernel(loader == kLoaderDirect ? k->direct : k->fn[loader],
+                                    (unsigned)grid, 1, 1, (unsigned)D.threads, 1, 1,
+                                    (unsigned)D.smem_bytes,
                                     reinterpret_cast<CUstream>(stream), args, nullptr);
   if (r) return cu_fail(r, "cuLaunchKernel");
   return CSD_OK;

@@ -912,6 +912,183 @@ __device__ __forceinline__ void register_chain(const csd_params& p) {
 }
 
 // ---------------------------------------------------------------------------
+// Direct kernels: one step from global memory, rows of any pitch
+// ---------------------------------------------------------------------------
+// Neither tensor copies nor 16-byte vectors reach rows whose pitch is not a
+// multiple of 16 bytes.  Here a warp owns PTS groups of 32 neighbouring
+// points of one row (lane l: columns l, l + 32, ...), so single-element loads
+// and stores are coalesced at any alignment, and walks Z.  Every "column"
+// (field, dy, dx) the body reads is loaded once, at its leading dz, and kept
+// in registers until its last dz (the body's tables); X and Y neighbours are
+// further loads that hit L1 (in 3-D the block's warps are neighbouring rows).
+// Each load is issued one row before its use, and occupancy hides the rest
+// (bringing planes to L2 ahead of that measured the same within 7 %).
+template <typename T_, int NIN_, int NOUT_, int RZ_, int RY_, int RX_, int NT_, int PTS_,
+          int REDUCE_, int NDIM_>
+struct DirectCfg {
+  typedef T_ T;
+  static constexpr int NIN = NIN_, NOUT = NOUT_, RZ = RZ_, RY = RY_, RX = RX_, NT = NT_;
+  static constexpr int PTS = PTS_, BC = CSD_BC_NONE, REDUCE = REDUCE_;
+  static constexpr int VEC = 1, RPY = 1, TEMPORAL = 1, ALIGN = 16 / (int)sizeof(T);
+  // 3-D: an item is the block's, a warp per row; else each warp has its own
+  static constexpr int TY = NDIM_ == 3 ? NT / 32 : 1, TX = 32 * PTS;
+  static constexpr int ROWS = 1, STAGES = 0, NSLOT = 0, HC = RZ, PADL = 0, BOXW = TX, BOXH = TY;
+  static constexpr int SMEM_BYTES = 0, BRICK_SHIFT = 0;
+};
+
+// A point's columns: v[column][k] is the value k planes above the column's
+// trailing one.
+template <class C, class Body>
+struct DirectView {
+  typedef typename C::T T;
+  const T (*v)[Body::WIN][C::PTS];
+  int e;
+  const double* scal;
+  const double* dyn;
+
+  __device__ __forceinline__ double scalar(int k) const { return scal[k]; }
+  __device__ __forceinline__ double dynamic(int k) const { return dyn[k]; }
+
+  template <int F, int DZ, int DY, int LO, int HI>
+  __device__ __forceinline__ Strip<T, LO, HI, 1> strip(int, int, int) const {
+    Strip<T, LO, HI, 1> s;
+#pragma unroll
+    for (int i = 0; i <= HI - LO; ++i) {
+      const int c = Body::col(F, DY, LO + i);   // < 0: read at another DZ or not at all
+      const int k = c < 0 ? -1 : DZ - Body::col_hi(c) + Body::col_len(c) - 1;
+      s.v[i] = c < 0 || k < 0 || k >= Body::col_len(c) ? T(0) : v[c][k][e];
+    }
+    return s;
+  }
+};
+
+// Rows narrower than a warp's points are walked 32 columns at a time.
+template <class C>
+struct NarrowCfg : C {
+  static constexpr int PTS = 1;
+};
+
+// One item's rows [z0, z0 + nrows) of array row y, columns xw + lane + 32 e.
+// NARROW: the lanes past the row's end read the last point's cells and store
+// nothing.
+template <class C, class Body, bool NARROW>
+__device__ __forceinline__ void direct_item(const csd_grid& g, int xw, int y, int z0, int nrows,
+                                            int xfirst) {
+  typedef typename C::T T;
+  constexpr int P = C::PTS, NC = Body::NCOL, NG = Body::NGRP, WIN = Body::WIN;
+  const int lane = threadIdx.x & 31;
+  const int hx = g.halo[2], nx = g.interior[2];
+  const long long pz = g.pitch_z, py = g.pitch_y;
+  const int x = xw + lane, zfirst = g.halo[0] + z0;
+  const double* scal = g.scalars;
+  const double* dyn = g.dyn;
+
+  T v[NC][WIN][P];   // the columns, oldest plane first
+  T nxt[NC][P];      // their next plane, in flight
+  const T* src[NG];  // row of a group (field, dy, leading dz) in plane 0
+#pragma unroll
+  for (int q = 0; q < NG; ++q)
+    src[q] = reinterpret_cast<const T*>(g.in[Body::grp_f(q)]) + (y + Body::grp_dy(q)) * py + x;
+
+  // column c of point e at its leading dz over row z
+  auto load = [&](int c, int e, int z) -> T {
+    const int q = Body::col_grp(c);
+    const int past = NARROW ? max(x + 32 * e - (hx + nx - 1), 0) : 0;
+    return __ldg(src[q] + (z + Body::grp_hi(q)) * pz + (Body::col_dx(c) + 32 * e - past));
+  };
+
+  T* dst[C::NOUT];
+#pragma unroll
+  for (int f = 0; f < C::NOUT; ++f)
+    dst[f] = reinterpret_cast<T*>(g.out[f]) + zfirst * pz + y * py + x;
+  bool mine[P];   // points this item stores (a warp moved left re-reads some)
+#pragma unroll
+  for (int e = 0; e < P; ++e) mine[e] = x + 32 * e >= xfirst && x + 32 * e < hx + nx;
+
+  // the planes before the first row's leading one
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+#pragma unroll
+    for (int k = 0; k < WIN; ++k)
+#pragma unroll
+      for (int e = 0; e < P; ++e)
+        v[c][k][e] = k + 1 < Body::col_len(c) ? load(c, e, zfirst - (Body::col_len(c) - 1 - k)) : T(0);
+  }
+#pragma unroll
+  for (int c = 0; c < NC; ++c)
+#pragma unroll
+    for (int e = 0; e < P; ++e) nxt[c][e] = load(c, e, zfirst);
+
+  double red_acc = 0.0;
+  const int zlast = zfirst + nrows - 1;
+#pragma unroll WIN
+  for (int z = zfirst; z <= zlast; ++z) {
+#pragma unroll
+    for (int c = 0; c < NC; ++c)
+#pragma unroll
+      for (int e = 0; e < P; ++e) v[c][Body::col_len(c) - 1][e] = nxt[c][e];
+    const int zn = min(z + 1, zlast);   // the last row loads its own columns again
+#pragma unroll
+    for (int c = 0; c < NC; ++c)
+#pragma unroll
+      for (int e = 0; e < P; ++e) nxt[c][e] = load(c, e, zn);
+#pragma unroll
+    for (int e = 0; e < P; ++e) {
+      OutPack<T, C::NOUT, 1> o;
+      const DirectView<C, Body> view{v, e, scal, dyn};
+      Body::template compute<C>(view, 0, 0, 0, o);
+      if constexpr (C::REDUCE) {
+        const double w = (double)o.v[0][0];
+        if (mine[e]) red_acc = (w != w || w > red_acc) ? w : red_acc;
+      } else {
+#pragma unroll
+        for (int f = 0; f < C::NOUT; ++f)
+          if (mine[e]) dst[f][32 * e] = o.v[f][0];
+      }
+    }
+#pragma unroll
+    for (int f = 0; f < C::NOUT; ++f) dst[f] += pz;
+#pragma unroll
+    for (int c = 0; c < NC; ++c)
+#pragma unroll
+      for (int k = 0; k + 1 < Body::col_len(c); ++k)
+#pragma unroll
+        for (int e = 0; e < P; ++e) v[c][k][e] = v[c][k + 1][e];
+  }
+  if constexpr (C::REDUCE) {
+    for (int o = 16; o > 0; o >>= 1) {
+      const double w = __shfl_down_sync(0xffffffffu, red_acc, o);
+      red_acc = (w != w || w > red_acc) ? w : red_acc;
+    }
+    if (lane == 0 && g.red) atomic_max_nonneg(g.red, red_acc);
+  }
+}
+
+template <class C, class Body>
+__device__ __forceinline__ void direct_step(const csd_params& p) {
+  const csd_grid& g = p.g;
+  constexpr int NW = C::NT / 32, PER = C::TY > 1 ? 1 : NW;   // items a block works on at once
+  const int warp = threadIdx.x >> 5;
+  for (int item = blockIdx.x * PER + (PER > 1 ? warp : 0); item < g.items; item += gridDim.x * PER) {
+    int tx, ty, z0, nrows;
+    csd_item_place(&g, item, &tx, &ty, &z0, &nrows);
+    const int hx = g.halo[2], nx = g.interior[2], hy = g.halo[1], ny = g.interior[1];
+    const int y = g.ybase + ty * C::TY + (C::TY > 1 ? warp : 0);
+    if (y >= hy + ny) continue;
+    // the last warp of a row moves left so that every lane has a point
+    const int xfirst = hx + tx * C::TX;
+    const int xw = max(min(xfirst, hx + nx - C::TX), hx);
+    if (nx >= C::TX) {
+      direct_item<C, Body, false>(g, xw, y, z0, nrows, xfirst);
+    } else {
+#pragma unroll 1
+      for (int xo = hx; xo < hx + nx; xo += 32)
+        direct_item<NarrowCfg<C>, Body, true>(g, xo, y, z0, nrows, xo);
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
 // The engine
 // ---------------------------------------------------------------------------
 template <class C, class Body, bool BATCHED>

@@ -191,16 +191,21 @@ class _ShiftClasses:
         return cid
 
 
-def emit_body(kernel: KernelOp) -> str:
-    """Device functor for the kernel's stencil body(ies)."""
-    name = kernel.kernel_name.data
+def emit_body(kernel: KernelOp, vec: int | None = None, suffix: str = "",
+              members: list | None = None) -> str:
+    """Device functor ``Body_<name><suffix>`` for the kernel's stencil
+    body(ies): ``vec`` points per unit (default: the kernel's own), with
+    ``members`` as further member declarations."""
+    name = kernel.kernel_name.data + suffix
     ndim = kernel.ndim.data
     dtype = kernel.dtype.data
     field_t = "f32" if dtype in ("float32", "fp32") else "f64"
     store_t = "float" if field_t == "f32" else "double"
     params = engine_params(kernel)
-    vec = params["VEC"]   # X points per unit (engine Cfg::VEC; 16 bytes unless widened)
-    rpy = params["RPY"]   # Y rows per thread (engine Cfg::RPY)
+    # X points per unit (engine Cfg::VEC; 16 bytes unless widened) and Y rows
+    # per thread (engine Cfg::RPY)
+    rpy = params["RPY"] if vec is None else 1
+    vec = vec or params["VEC"]
     accesses = [tuple(a.data for a in acc) for acc in kernel.accesses.data]
     acc_info = [_internal_offsets(ndim, offs) + (f,) for f, *offs in accesses]  # (dz, dy, dx, f)
     # strip groups: (field, dz, dy of the unit's row 0) -> X range, over all rows
@@ -217,6 +222,7 @@ def emit_body(kernel: KernelOp) -> str:
     unroll = 4 if (len(gkeys) <= 8 and rpy == 1 and body_lines <= 48) else 0
     out = [f"struct Body_{name} {{",
            f"  static constexpr int UNROLL = {unroll};",
+           *[f"  {m}" for m in members or []],
            "  template <class C, class View>",
            "  __device__ __forceinline__ static void compute(const View& t, int r, int y,",
            "                                                 int x, csd::OutPack<typename C::T, "
@@ -319,6 +325,114 @@ def emit_body(kernel: KernelOp) -> str:
 CHAIN_THREADS = 128   # four independent warps per block of a register chain
 
 
+DIRECT_THREADS = 256
+
+
+def direct_columns(kernel: KernelOp) -> dict:
+    """The columns a direct kernel keeps per point (engine.cuh ``DirectCfg``):
+    distinct ``(field, dy, dx)`` with the range of dz the body reads there."""
+    ndim = kernel.ndim.data
+    cols: dict[tuple, list] = {}
+    for f, *offs in (tuple(a.data for a in acc) for acc in kernel.accesses.data):
+        dz, dy, dx = _internal_offsets(ndim, offs)
+        cols.setdefault((f, dy, dx), []).append(dz)
+    return {k: (min(v), max(v)) for k, v in sorted(cols.items())}
+
+
+def direct_plan(kernel: KernelOp) -> tuple:
+    """``(points per lane, blocks per SM)`` of the kernel's direct form, or
+    ``(0, 0)`` where it has none: fused boundary fills, chains and bricks keep
+    the ring, and so do long bodies, which share values between neighbouring
+    points, and columns that do not fit the registers.
+
+    Four points per lane pay where the columns and their next plane leave
+    three blocks per SM (7-point 301 x 411 x 523, FP32 / FP64 us: four points
+    130 / 212, two 145 / 240, one 188 / 263; the ring's per-element copies 402
+    / 458).  Longer bodies take two (RK4 stage of a radius-2 operator, 1537 x
+    2049 FP64: 25 us, four points 35; 27-point box 301 x 311 x 323 FP64: 185,
+    one point 242, the ring 274)."""
+    p = engine_params(kernel)
+    lines = sum(len(prog.data) for prog in kernel.ssa_body.data)
+    if p["BRICK"] or p["TEMPORAL"] != 1 or p["BC"] != BC_CODES["none"] or lines > 100:
+        return (0, 0)
+    words = sum(hi - lo + 2 for lo, hi in direct_columns(kernel).values()) * p["dtype_bytes"] // 4
+    points, blocks = ((4, 3) if words <= 24 and lines <= 16 else (2, 2) if words <= 72 else
+                      (1, 1) if words <= 144 else (0, 0))
+    return (points, p["OCCUPANCY"] or blocks) if points else (0, 0)
+
+
+def _table(name: str, args: str, rows: dict) -> str:
+    """A constexpr device lookup ``name(args)`` over ``rows`` {condition: value}."""
+    expr = "".join(f"{cond} ? {value} : " for cond, value in rows.items())
+    return f"__host__ __device__ static constexpr int {name}({args}) {{ return {expr}-1; }}"
+
+
+def _direct_members(kernel: KernelOp) -> list:
+    """Column and group tables of a direct body.  A group is the columns
+    loaded through one row pointer (field, dy, leading dz)."""
+    cols = direct_columns(kernel)
+    groups: list = []
+    for (f, dy, dx), (lo, hi) in cols.items():
+        if (f, dy, hi) not in groups:
+            groups.append((f, dy, hi))
+    cl = list(cols.items())
+
+    def by_col(fn):
+        return {f"c == {i}": fn(*cl[i][0], *cl[i][1]) for i in range(len(cl))}
+
+    def by_grp(fn):
+        return {f"q == {i}": fn(*g) for i, g in enumerate(groups)}
+
+    return [
+        f"static constexpr int NCOL = {len(cl)}, NGRP = {len(groups)}, "
+        f"WIN = {max(hi - lo + 1 for lo, hi in cols.values())};",
+        _table("col", "int f, int dy, int dx",
+               {f"f == {f} && dy == {dy} && dx == {dx}": i
+                for i, ((f, dy, dx), _) in enumerate(cl)}),
+        _table("col_dx", "int c", by_col(lambda f, dy, dx, lo, hi: dx)),
+        _table("col_hi", "int c", by_col(lambda f, dy, dx, lo, hi: hi)),
+        _table("col_len", "int c", by_col(lambda f, dy, dx, lo, hi: hi - lo + 1)),
+        _table("col_grp", "int c", by_col(lambda f, dy, dx, lo, hi: groups.index((f, dy, hi)))),
+        _table("grp_f", "int q", by_grp(lambda f, dy, hi: f)),
+        _table("grp_dy", "int q", by_grp(lambda f, dy, hi: dy)),
+        _table("grp_hi", "int q", by_grp(lambda f, dy, hi: hi)),
+    ]
+
+
+def _emit_direct(kernel: KernelOp) -> list:
+    """The ``<name>_direct`` kernel and its descriptor (rows of any pitch)."""
+    name = kernel.kernel_name.data
+    p = engine_params(kernel)
+    points, min_blocks = direct_plan(kernel)
+    c = f"Cfg_{name}_direct"
+    return [
+        emit_body(kernel, 1, "_direct", _direct_members(kernel)),
+        f"typedef csd::DirectCfg<{p['T']}, {p['NIN']}, {p['NOUT']}, {p['RZ']}, {p['RY']}, "
+        f"{p['RX']}, {DIRECT_THREADS}, {points}, {p['REDUCE']}, {p['ndim']}> {c};",
+        f'extern "C" __global__ void __launch_bounds__({DIRECT_THREADS}, {min_blocks})',
+        f"{name}_direct(const __grid_constant__ csd_params p) {{",
+        f"  csd::direct_step<{c}, Body_{name}_direct>(p);",
+        "}",
+        _descriptor(f"{name}_direct_desc", c, p, 0, min_blocks, 0),
+        "",
+    ]
+
+
+def _descriptor(symbol: str, c: str, p: dict, zchunk: int, min_blocks: int,
+                brick_tma: int, smem: str | None = None) -> str:
+    """``csd_kernel_desc`` of configuration type ``c``."""
+    nout = "0" if p["REDUCE"] else f"{c}::NOUT"
+    return "\n".join([
+        f'extern "C" __device__ const csd_kernel_desc {symbol} = {{',
+        f"  CSD_DESC_MAGIC, {p['ndim']}, {c}::NIN, {nout}, (int)sizeof({c}::T),",
+        f"  {c}::RZ * {c}::TEMPORAL, {c}::RY * {c}::TEMPORAL, {c}::RX * {c}::TEMPORAL,",
+        f"  {c}::ROWS, {c}::TY, {c}::TX, {c}::VEC, {c}::NT, {c}::STAGES, {c}::NSLOT,",
+        f"  {c}::HC * {c}::TEMPORAL, {c}::PADL, {c}::BOXW, {c}::BOXH, "
+        f"{smem or f'{c}::SMEM_BYTES'},",
+        f"  {zchunk}, {c}::TEMPORAL, {c}::BC, {min_blocks}, {c}::ALIGN,",
+        f"  {p['NSCAL']}, {p['NDYN']}, {p['REDUCE']}, {c}::BRICK_SHIFT, {brick_tma}}};"])
+
+
 def _internal_radius(ndim: int, radius) -> tuple[int, int, int]:
     r = list(radius)
     if ndim == 3:
@@ -364,6 +478,7 @@ def engine_params(kernel: KernelOp) -> dict:
         "REDUCE": kernel.reduce_max.data if kernel.reduce_max is not None else 0,
         "BRICK": _brick_code(kernel, ndim),
         "RPY": int(hints.get("rpy", 1)),
+        "OCCUPANCY": int(hints.get("occupancy", 0)),   # a caller's blocks per SM (0: none)
         # points per lane of a register chain (0: the ring engine)
         "CHAIN": int(hints.get("register_chain", 0)),
         "VEC": int(hints.get("register_chain", 0)
@@ -442,19 +557,14 @@ def emit_cuda(module: ModuleOp, preamble: bool = True) -> str:
             parts.append(f"  csd::{entry}<Cfg_{name}_{suffix}, Body_{name}>(p);")
             parts.append("}")
         c = f"Cfg_{name}_tma"
-        parts.append(f'extern "C" __device__ const csd_kernel_desc {name}_desc = {{')
-        nout_desc = "0" if p["REDUCE"] else f"{c}::NOUT"
-        parts.append(f"  CSD_DESC_MAGIC, {p['ndim']}, {c}::NIN, {nout_desc}, (int)sizeof({c}::T),")
-        parts.append(f"  {c}::RZ * {c}::TEMPORAL, {c}::RY * {c}::TEMPORAL, {c}::RX * {c}::TEMPORAL,")
-        parts.append(f"  {c}::ROWS, {c}::TY, {c}::TX, {c}::VEC, {c}::NT, {c}::STAGES, {c}::NSLOT,")
         # both entries launch with one shared-memory size: the larger one
         smem = (f"({c}::SMEM_BYTES > Cfg_{name}_ldg::SMEM_BYTES ? {c}::SMEM_BYTES : "
                 f"Cfg_{name}_ldg::SMEM_BYTES)")
-        parts.append(f"  {c}::HC * {c}::TEMPORAL, {c}::PADL, {c}::BOXW, {c}::BOXH, {smem},")
-        parts.append(f"  {p['ZCHUNK']}, {c}::TEMPORAL, {c}::BC, {p['MINB']}, {c}::ALIGN,")
-        parts.append(f"  {p['NSCAL']}, {p['NDYN']}, {p['REDUCE']}, {c}::BRICK_SHIFT, "
-                     f"{1 if brick_tma else 0}}};")
+        parts.append(_descriptor(f"{name}_desc", c, p, p["ZCHUNK"], p["MINB"],
+                                 1 if brick_tma else 0, smem))
         parts.append("")
+        if direct_plan(kernel)[0]:
+            parts.extend(_emit_direct(kernel))
     return "\n".join(parts) + "\n"
 
 
