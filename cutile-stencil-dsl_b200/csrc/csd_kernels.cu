@@ -269,15 +269,22 @@ extern "C" int csd_from_bricks(const void* bricked, int brick, const csd_field* 
 // ---------------------------------------------------------------------------
 // FP64 reductions over the interior of a field (mass, energy, residual, max)
 //
-// Deterministic: pass 1 gives CTA b the interior rows [b*R/G, (b+1)*R/G) of
-// the (Z*Y) x X row grid; each thread accumulates its elements in a fixed
-// order in FP64, then a fixed-shape tree reduces the CTA's threads into
-// partials[b].  Pass 2 (one CTA) reduces partials[0..G) the same way.  The
-// result depends on G, never on scheduling.
+// Deterministic: interior rows are cut into segments of RED_SEG elements, and
+// pass 1 gives CTA b the segments [b*S/G, (b+1)*S/G), its warps taking them in
+// turn.  A lane adds its elements in RED_ILP independent FP64 sums in a fixed
+// order, and a fixed-shape tree reduces lanes and warps into partials[b].
+// Pass 2 (one CTA) reduces partials[0..G) the same way.  The result depends on
+// G, never on scheduling.  Bound by HBM: RED_ILP loads per lane and 16 warps
+// per CTA keep enough of them in flight with two CTAs per SM (sum of a 300 x
+// 320 x 340 FP64 interior, 261 MB: 56 us, the difference of two 100; with a
+// row at a time per CTA of 256 threads 388 and 449; a 1-D
+// row, formerly one CTA's, 2^24 FP64: 10.9 ms -> 34 us).
 // ---------------------------------------------------------------------------
 namespace {
 
-constexpr int RED_THREADS = 256;
+constexpr int RED_THREADS = 512, RED_THREADS2 = 256;   // pass 1, pass 2
+constexpr int RED_ILP = 8;
+constexpr int RED_SEG = 1024;   // elements of a row segment
 
 template <int OP>
 __device__ __forceinline__ double red_combine(double a, double b) {
@@ -285,7 +292,7 @@ __device__ __forceinline__ double red_combine(double a, double b) {
   return a + b;
 }
 
-template <int OP>
+template <int OP, int THREADS>
 __device__ __forceinline__ double red_block(double v, double* sh) {
   // fixed-shape tree: warp shuffles, then the warp totals in order
   for (int o = 16; o > 0; o >>= 1) v = red_combine<OP>(v, __shfl_down_sync(0xffffffffu, v, o));
@@ -295,48 +302,88 @@ __device__ __forceinline__ double red_block(double v, double* sh) {
   double t = 0.0;
   if (threadIdx.x == 0) {
     t = sh[0];
-    for (int w = 1; w < RED_THREADS / 32; ++w) t = red_combine<OP>(t, sh[w]);
+    for (int w = 1; w < THREADS / 32; ++w) t = red_combine<OP>(t, sh[w]);
   }
   __syncthreads();
   return t;
 }
 
+// The reduced value of one element.
+template <int OP>
+__device__ __forceinline__ double red_value(double va, double vb) {
+  if (OP == CSD_RED_SUM) return va;
+  if (OP == CSD_RED_SUMSQ) return va * va;
+  if (OP == CSD_RED_MAXABS) return fabs(va);
+  const double d = va - vb;
+  return OP == CSD_RED_DIFF_SUMSQ ? d * d : fabs(d);
+}
+
 template <typename T, int OP>
-__global__ void __launch_bounds__(RED_THREADS) reduce_pass1(const T* a, const T* b, long long d0,
-                                                            long long d1, long long d2, int h0,
-                                                            int h1, int h2, double* partials) {
+__global__ void __launch_bounds__(RED_THREADS, 2) reduce_pass1(const T* a, const T* b,
+                                                               long long d0, long long d1,
+                                                               long long d2, int h0, int h1,
+                                                               int h2, double* partials) {
   __shared__ double sh[RED_THREADS / 32];
+  constexpr bool kDiff = OP == CSD_RED_DIFF_SUMSQ || OP == CSD_RED_DIFF_MAXABS;
   const long long ny = d1 - 2 * h1, nx = d2 - 2 * h2;
-  const long long rows = (d0 - 2 * h0) * ny;
-  const long long r0 = rows * blockIdx.x / gridDim.x, r1 = rows * (blockIdx.x + 1) / gridDim.x;
-  double acc = 0.0;
-  for (long long r = r0; r < r1; ++r) {
-    const long long z = r / ny + h0, y = r % ny + h1;
-    const long long base = (z * d1 + y) * d2 + h2;
-    for (long long x = threadIdx.x; x < nx; x += RED_THREADS) {
-      const double va = (double)a[base + x];
-      double v;
-      if (OP == CSD_RED_SUM) v = va;
-      else if (OP == CSD_RED_SUMSQ) v = va * va;
-      else if (OP == CSD_RED_MAXABS) v = fabs(va);
-      else {
-        const double d = va - (double)b[base + x];
-        v = (OP == CSD_RED_DIFF_SUMSQ) ? d * d : fabs(d);
-      }
-      acc = red_combine<OP>(acc, v);
+  const long long nseg = (nx + RED_SEG - 1) / RED_SEG;
+  const long long segs = (d0 - 2 * h0) * ny * nseg;
+  const long long s0 = segs * blockIdx.x / gridDim.x, s1 = segs * (blockIdx.x + 1) / gridDim.x;
+  const int lane = threadIdx.x & 31;
+  constexpr int NW = RED_THREADS / 32;
+  // (z, y, seg) of the warp's first segment and the step to its next one
+  long long i = s0 + (threadIdx.x >> 5);
+  long long seg = i % nseg, z = i / nseg / ny, y = i / nseg % ny;
+  const long long dseg = NW % nseg, dz = NW / nseg / ny, dy = NW / nseg % ny;
+  double acc[RED_ILP];
+#pragma unroll
+  for (int k = 0; k < RED_ILP; ++k) acc[k] = 0.0;
+  for (; i < s1; i += NW) {
+    const long long base = ((z + h0) * d1 + y + h1) * d2 + h2 + seg * RED_SEG;
+    const int n = (int)min((long long)RED_SEG, nx - seg * RED_SEG);
+    const T* pa = a + base;
+    const T* pb = kDiff ? b + base : nullptr;
+    int x = lane;
+    for (; x + 32 * (RED_ILP - 1) < n; x += 32 * RED_ILP) {
+      double v[RED_ILP];
+#pragma unroll
+      for (int k = 0; k < RED_ILP; ++k)
+        v[k] = red_value<OP>((double)pa[x + 32 * k], kDiff ? (double)pb[x + 32 * k] : 0.0);
+#pragma unroll
+      for (int k = 0; k < RED_ILP; ++k) acc[k] = red_combine<OP>(acc[k], v[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < RED_ILP; ++k)
+      if (x + 32 * k < n)
+        acc[k] = red_combine<OP>(acc[k], red_value<OP>((double)pa[x + 32 * k],
+                                                       kDiff ? (double)pb[x + 32 * k] : 0.0));
+    seg += dseg;
+    y += dy;
+    z += dz;
+    if (seg >= nseg) {
+      seg -= nseg;
+      ++y;
+    }
+    if (y >= ny) {
+      y -= ny;
+      ++z;
     }
   }
-  const double t = red_block<OP>(acc, sh);
+#pragma unroll
+  for (int w = RED_ILP / 2; w > 0; w >>= 1)
+#pragma unroll
+    for (int k = 0; k < w; ++k) acc[k] = red_combine<OP>(acc[k], acc[k + w]);
+  const double t = red_block<OP, RED_THREADS>(acc[0], sh);
   if (threadIdx.x == 0) partials[blockIdx.x] = t;
 }
 
 template <int OP>
-__global__ void __launch_bounds__(RED_THREADS) reduce_pass2(const double* partials, int n,
-                                                            double* result) {
-  __shared__ double sh[RED_THREADS / 32];
+__global__ void __launch_bounds__(RED_THREADS2) reduce_pass2(const double* partials, int n,
+                                                             double* result) {
+  __shared__ double sh[RED_THREADS2 / 32];
   double acc = 0.0;
-  for (int i = threadIdx.x; i < n; i += RED_THREADS) acc = red_combine<OP>(acc, partials[i]);
-  const double t = red_block<OP>(acc, sh);
+  for (int i = threadIdx.x; i < n; i += RED_THREADS2) acc = red_combine<OP>(acc, partials[i]);
+  const double t = red_block<OP, RED_THREADS2>(acc, sh);
   if (threadIdx.x == 0) *result = t;
 }
 
@@ -347,7 +394,7 @@ int reduce_t(const csd_field* a, const csd_field* b, const long long d[3], const
   const T* pb = b ? reinterpret_cast<const T*>(b->ptr) : nullptr;
   reduce_pass1<T, OP><<<nblocks, RED_THREADS, 0, s>>>(pa, pb, d[0], d[1], d[2], h[0], h[1], h[2],
                                                       partials);
-  reduce_pass2<OP><<<1, RED_THREADS, 0, s>>>(partials, nblocks, result);
+  reduce_pass2<OP><<<1, RED_THREADS2, 0, s>>>(partials, nblocks, result);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? CSD_OK : csd_internal_fail(CSD_ELAUNCH, cudaGetErrorString(e));
 }
