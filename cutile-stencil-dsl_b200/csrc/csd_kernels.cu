@@ -136,58 +136,88 @@ extern "C" int csd_apply_boundary(const csd_field* f, const int* halo, int bc, d
 // bricks of B^nd elements, bricks in row-major order over the brick grid
 // (ceil(n / B) per dim) and each brick row-major inside: the reference's
 // to_bricks reshape/transpose (multigpu_emitter.py:370-408), padded cells
-// zero.  One thread per element; to_bricks walks the bricked order (writes
-// coalesced, reads in runs of B), from_bricks the flat order.
+// zero.  A warp takes a segment of one array row: its brick offset is worked
+// out once, lanes run along X, and an element costs shifts and adds.  Bound by
+// HBM: 300 x 320 x 370 FP64, B = 8, 284 MB each way: to_bricks 221 -> 107 us,
+// from_bricks 177 -> 110 (one thread per element, with 64-bit divisions).
 // ---------------------------------------------------------------------------
 namespace {
 
-__device__ __forceinline__ long long brick_off(long long z, long long y, long long x, int nd, int s,
-                                               long long nby, long long nbx) {
+constexpr int BRICK_SEG = 1024;   // elements of a row segment
+
+// TO: flat -> bricked over the padded rows (zeros past the array); else
+// bricked -> flat over the array's rows.  r0 x r1 rows of r2 elements are
+// walked; `I` counts their segments.
+template <typename T, typename I, bool TO>
+__global__ void __launch_bounds__(256) brick_rows_kernel(const T* __restrict__ src,
+                                                         T* __restrict__ dst, long long n0,
+                                                         long long n1, long long n2, I r0, I r1,
+                                                         long long r2, int nd, int s,
+                                                         long long nb1, long long nb2) {
   const long long m = (1ll << s) - 1;
-  if (nd == 3)
-    return ((((z >> s) * nby + (y >> s)) * nbx + (x >> s)) << (3 * s)) + ((z & m) << (2 * s)) +
-           ((y & m) << s) + (x & m);
-  if (nd == 2) return ((((y >> s) * nbx + (x >> s)) << (2 * s)) + ((y & m) << s) + (x & m));
-  return x;
-}
-
-template <typename T>
-__global__ void to_bricks_kernel(const T* __restrict__ flat, T* __restrict__ bricked, long long n0,
-                                 long long n1, long long n2, int nd, int s, long long nb0,
-                                 long long nb1, long long nb2) {
-  const long long B = 1ll << s;
-  const long long total = nb0 * nb1 * nb2 * (nd == 3 ? B * B * B : nd == 2 ? B * B : B);
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
-       e += (long long)gridDim.x * blockDim.x) {
-    long long z = 0, y = 0, x;
-    const long long m = B - 1;
-    if (nd == 3) {
-      const long long b = e >> (3 * s), r = e & ((1ll << (3 * s)) - 1);
-      x = ((b % nb2) << s) + (r & m);
-      y = (((b / nb2) % nb1) << s) + ((r >> s) & m);
-      z = ((b / (nb2 * nb1)) << s) + (r >> (2 * s));
-    } else if (nd == 2) {
-      const long long b = e >> (2 * s), r = e & ((1ll << (2 * s)) - 1);
-      x = ((b % nb2) << s) + (r & m);
-      y = ((b / nb2) << s) + (r >> s);
-    } else {
-      x = e;
+  const I nseg = (I)((r2 + BRICK_SEG - 1) / BRICK_SEG);
+  const I units = r0 * r1 * nseg;
+  const int lane = threadIdx.x & 31;
+  const I warps = (I)gridDim.x * (blockDim.x >> 5);
+  for (I u = (I)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); u < units; u += warps) {
+    const I row = u / nseg;
+    const long long x0 = (long long)(u - row * nseg) * BRICK_SEG;
+    const long long z = (long long)(row / r1), y = (long long)(row % r1);
+    // element x of the row is at brow + ((x >> s) << (nd s)) + (x & m)
+    long long brow = 0;
+    if (nd == 3)
+      brow = ((((z >> s) * nb1 + (y >> s)) * nb2) << (3 * s)) + ((z & m) << (2 * s)) +
+             ((y & m) << s);
+    else if (nd == 2)
+      brow = (((y >> s) * nb2) << (2 * s)) + ((y & m) << s);
+    const long long frow = (z * n1 + y) * n2;
+    const bool in = z < n0 && y < n1;
+    const int n = (int)min((long long)BRICK_SEG, r2 - x0);
+    for (int k = lane; k < n; k += 128) {
+      T v[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const long long x = x0 + k + 32 * q;
+        v[q] = T(0);
+        if (k + 32 * q < n) {
+          if (TO) {
+            if (in && x < n2) v[q] = src[frow + x];
+          } else {
+            v[q] = src[brow + ((x >> s) << (nd * s)) + (x & m)];
+          }
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const long long x = x0 + k + 32 * q;
+        if (k + 32 * q < n) {
+          if (TO)
+            dst[brow + ((x >> s) << (nd * s)) + (x & m)] = v[q];
+          else
+            dst[frow + x] = v[q];
+        }
+      }
     }
-    const bool in = z < n0 && y < n1 && x < n2;
-    bricked[e] = in ? flat[(z * n1 + y) * n2 + x] : T(0);
   }
 }
 
-template <typename T>
-__global__ void from_bricks_kernel(const T* __restrict__ bricked, T* __restrict__ flat, long long n0,
-                                   long long n1, long long n2, int nd, int s, long long nb1,
-                                   long long nb2) {
-  const long long total = n0 * n1 * n2;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
-       e += (long long)gridDim.x * blockDim.x) {
-    const long long x = e % n2, t = e / n2, y = t % n1, z = t / n1;
-    flat[e] = bricked[brick_off(z, y, x, nd, s, nb1, nb2)];
-  }
+template <typename T, bool TO>
+void launch_brick_rows(const void* src, void* dst, const long long n[3], const long long nb[3],
+                       int nd, int s, cudaStream_t st) {
+  long long r[3];
+  for (int i = 0; i < 3; ++i) r[i] = TO && i >= 3 - nd ? nb[i] << s : n[i];
+  const long long units = r[0] * r[1] * ((r[2] + BRICK_SEG - 1) / BRICK_SEG);
+  long long blocks = (units + 7) / 8;
+  if (blocks > 148 * 8) blocks = 148 * 8;
+  const T* from = static_cast<const T*>(src);
+  T* to = static_cast<T*>(dst);
+  if (units < (1ll << 30))
+    brick_rows_kernel<T, unsigned, TO><<<(int)blocks, 256, 0, st>>>(
+        from, to, n[0], n[1], n[2], (unsigned)r[0], (unsigned)r[1], r[2], nd, s, nb[1], nb[2]);
+  else
+    brick_rows_kernel<T, unsigned long long, TO><<<(int)blocks, 256, 0, st>>>(
+        from, to, n[0], n[1], n[2], (unsigned long long)r[0], (unsigned long long)r[1], r[2], nd,
+        s, nb[1], nb[2]);
 }
 
 // (n0, n1, n2) view, bricked dimensionality and brick-grid extents of a field
@@ -223,19 +253,11 @@ extern "C" int csd_to_bricks(const csd_field* flat, int brick, void* bricked, vo
   int rc = brick_geometry(flat, brick, n, nb, &nd, &s);
   if (rc) return rc;
   if (!bricked) return csd_internal_fail(CSD_EINVAL, "null bricked buffer");
-  const long long total = nb[0] * nb[1] * nb[2] * (nd == 3 ? (long long)brick * brick * brick
-                                                   : nd == 2 ? (long long)brick * brick : brick);
-  long long blocks = (total + 255) / 256;
-  if (blocks > 148 * 32) blocks = 148 * 32;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (flat->dtype == CSD_DTYPE_F64)
-    to_bricks_kernel<double><<<(int)blocks, 256, 0, st>>>(
-        static_cast<const double*>(flat->ptr), static_cast<double*>(bricked), n[0], n[1], n[2], nd,
-        s, nb[0], nb[1], nb[2]);
+    launch_brick_rows<double, true>(flat->ptr, bricked, n, nb, nd, s, st);
   else if (flat->dtype == CSD_DTYPE_F32)
-    to_bricks_kernel<float><<<(int)blocks, 256, 0, st>>>(
-        static_cast<const float*>(flat->ptr), static_cast<float*>(bricked), n[0], n[1], n[2], nd,
-        s, nb[0], nb[1], nb[2]);
+    launch_brick_rows<float, true>(flat->ptr, bricked, n, nb, nd, s, st);
   else
     return csd_internal_fail(CSD_EINVAL, "unsupported dtype");
   cudaError_t e = cudaGetLastError();
@@ -248,18 +270,11 @@ extern "C" int csd_from_bricks(const void* bricked, int brick, const csd_field* 
   int rc = brick_geometry(flat, brick, n, nb, &nd, &s);
   if (rc) return rc;
   if (!bricked) return csd_internal_fail(CSD_EINVAL, "null bricked buffer");
-  const long long total = n[0] * n[1] * n[2];
-  long long blocks = (total + 255) / 256;
-  if (blocks > 148 * 32) blocks = 148 * 32;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (flat->dtype == CSD_DTYPE_F64)
-    from_bricks_kernel<double><<<(int)blocks, 256, 0, st>>>(
-        static_cast<const double*>(bricked), static_cast<double*>(flat->ptr), n[0], n[1], n[2], nd,
-        s, nb[1], nb[2]);
+    launch_brick_rows<double, false>(bricked, flat->ptr, n, nb, nd, s, st);
   else if (flat->dtype == CSD_DTYPE_F32)
-    from_bricks_kernel<float><<<(int)blocks, 256, 0, st>>>(
-        static_cast<const float*>(bricked), static_cast<float*>(flat->ptr), n[0], n[1], n[2], nd,
-        s, nb[1], nb[2]);
+    launch_brick_rows<float, false>(bricked, flat->ptr, n, nb, nd, s, st);
   else
     return csd_internal_fail(CSD_EINVAL, "unsupported dtype");
   cudaError_t e = cudaGetLastError();

@@ -181,3 +181,22 @@ def test_brick_sized_halo_starts_the_interior_on_a_brick(dtype, loader):
     mask = np.ones(shape, bool)
     mask[inner] = False
     assert np.all(got[mask] == 7.0)
+
+
+@pytest.mark.parametrize("shape,brick", [((5,), 4), ((3000,), 64), ((2, 1030), 8), ((17, 1023), 4),
+                                         ((3, 5, 1025), 16), ((9, 8, 7), 8), ((1, 1, 2049), 4)])
+@pytest.mark.parametrize("dtype", ["float32", "float64"])
+def test_conversions_over_row_segments(shape, brick, dtype):
+    """Rows shorter and longer than a segment, padded bricks, every
+    dimensionality: the bricked form is the oracle's and converts back."""
+    import torch
+
+    from cutile.runtime import native
+
+    u = np.random.default_rng(1).standard_normal(shape).astype(dtype)
+    t = torch.from_numpy(u).cuda()
+    b = native.to_bricks(t, brick)
+    assert np.array_equal(b.cpu().numpy(), O.to_bricks(u, brick))
+    out = torch.full_like(t, float("nan"))
+    native.from_bricks(b, shape, brick, out=out)
+    assert np.array_equal(out.cpu().numpy(), u)
