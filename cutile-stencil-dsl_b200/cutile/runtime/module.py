@@ -36,6 +36,7 @@ class StencilProgram:
         self.cubin = cubin
         self.cubin_sha256 = cubin_sha256
         self._modules: dict[int, native.NativeModule] = {}
+        self._plans = native.LaunchPlans()
         self._lock = threading.Lock()
 
     # -- loading -------------------------------------------------------------
@@ -86,6 +87,8 @@ class StencilProgram:
     # -- entry points --------------------------------------------------------
     def scalar_values(self, scalars: dict | None) -> list:
         names = self.spec.get("scalars", [])
+        if not names and not scalars:
+            return []
         scalars = scalars or {}
         missing = [n for n in names if n not in scalars]
         if missing:
@@ -106,17 +109,16 @@ class StencilProgram:
         that runs out stops its CTA and sets the device error word
         (``native.error_word``).  ``withhold_chunk`` is the failure-test hook
         of ``csd_launch_opts`` (one input chunk of CTA 0 is never requested)."""
-        self._check(list(inputs) + list(outputs), "stencil")
-        if len(inputs) != self.spec["inputs"] or len(outputs) != self.spec["outputs"]:
-            raise TypeError(f"launch_{self.spec['name']} takes {self.spec['inputs']} input(s) and "
-                            f"{self.spec['outputs']} output(s)")
-        for o in outputs:
-            for i in inputs:
-                if o.data_ptr() == i.data_ptr():
-                    raise ValueError("outputs must not alias inputs (the kernel reads neighbours)")
-        native.launch(self.kernel(which), inputs, outputs, self.spec["halo"], stream,
+        def check():
+            self._check(list(inputs) + list(outputs), "stencil")
+            if len(inputs) != self.spec["inputs"] or len(outputs) != self.spec["outputs"]:
+                raise TypeError(f"launch_{self.spec['name']} takes {self.spec['inputs']} input(s) "
+                                f"and {self.spec['outputs']} output(s)")
+
+        native.launch(lambda: self.kernel(which), inputs, outputs, self.spec["halo"], stream,
+                      plans=self._plans, kind=which, check_fields=check, distinct=True,
                       zchunk=zchunk, grid=grid, loader=loader,
-                      scalars=self.scalar_values(scalars), dyn=dyn, red=red, bc_odd=bc_odd,
+                      scalars=self.scalar_values(scalars), dyn=dyn, red=red, bc_odd=tuple(bc_odd),
                       timeout_ns=timeout_ns, withhold_chunk=withhold_chunk)
 
     def step(self, inputs, outputs, stream=None, *, scalars: dict | None = None, **kw) -> None:
@@ -124,9 +126,10 @@ class StencilProgram:
         ``out = stencil(apply_boundary(in))`` without writing the inputs' halos."""
         if "fused_bc" not in self.spec["kernels"]:
             raise ValueError(f"{self.spec['name']} declares no boundary condition")
-        self._check(list(inputs) + list(outputs), "stencil")
         bc = self.spec["boundary"] or {}
-        native.launch(self.kernel("fused_bc"), inputs, outputs, self.spec["halo"], stream,
+        native.launch(lambda: self.kernel("fused_bc"), inputs, outputs, self.spec["halo"], stream,
+                      plans=self._plans, kind="fused_bc",
+                      check_fields=lambda: self._check(list(inputs) + list(outputs), "stencil"),
                       bc_value=float(bc.get("value", 0.0)),
                       scalars=self.scalar_values(scalars), **kw)
 

@@ -29,6 +29,7 @@ class RKProgram:
         self.table = stage_table(spec["method"])
         self._modules: dict = {}
         self._lock = threading.Lock()
+        self._plans = native.LaunchPlans()
         self._work: dict = {}
         self._dt: dict = {}
         self.bc_odd: tuple = ()
@@ -111,8 +112,9 @@ class RKProgram:
         halo = self.spec["halo"]
         for k in range(len(self.table)):
             inputs, outputs = self.stage_io(k, bufs, tuple(fields[m:]) + tuple(aux))
-            native.launch(self.kernel(k), inputs, outputs, halo, stream, scalars=sv, dyn=dyn,
-                          bc_odd=self.bc_odd, bc_value=self.bc_value)
+            native.launch(lambda: self.kernel(k), inputs, outputs, halo, stream,  # noqa: B023
+                          plans=self._plans, kind=k, scalars=sv, dyn=dyn,
+                          bc_odd=tuple(self.bc_odd), bc_value=self.bc_value)
         last_out = self.table[-1][7]
         if last_out != "u":
             inner = tuple(slice(h, s - h) for h, s in zip(halo, state[0].shape))
