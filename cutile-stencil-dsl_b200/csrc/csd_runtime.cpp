@@ -570,10 +570,8 @@ static bool is_register_chain(const csd_kernel_desc& D) { return D.temporal > 1 
 static bool is_direct(const csd_kernel_desc& D) {
   return D.temporal == 1 && D.nslot == 0 && D.threads > 0;
 }
-// An item of theirs is a warp's (a direct 3-D kernel's: the block's).
-static int warps_per_item(const csd_kernel_desc& D) {
-  return is_register_chain(D) || (is_direct(D) && D.tile_y == 1) ? 1 : D.threads / 32;
-}
+// An item of theirs is a warp's, or in 3-D the block's.
+static int warps_per_item(const csd_kernel_desc& D) { return D.ndim < 3 ? 1 : D.threads / 32; }
 
 // Rows per item of a register chain (engine.cuh ChainCfg: one warp per item).
 // An item of r rows takes r + lead row times; a row's time grows slowly with
@@ -619,7 +617,8 @@ int csd_plan_items(const csd_kernel_desc* D, long long slots, int zchunk_req, cs
   if (is_register_chain(*D) && zchunk_req <= 0)
     // lead: 2 T RZ input rows, T steps of skew, and about four rows' time
     // before the first input arrives
-    zchunk = chain_rows(columns, nz, 2ll * D->rz + D->temporal + 4, D->threads / 32, slots);
+    zchunk = chain_rows(columns, nz, 2ll * D->rz + D->temporal + 4,
+                        D->threads / 32 / warps_per_item(*D), slots);
   // a direct kernel's lead is the 2 RZ rows it reads again; the split that suits
   // a chain measured within 5 % of the best of 8 to 301 rows here too
   if (is_direct(*D) && zchunk_req <= 0)

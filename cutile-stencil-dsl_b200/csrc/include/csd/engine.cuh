@@ -912,6 +912,263 @@ __device__ __forceinline__ void register_chain(const csd_params& p) {
 }
 
 // ---------------------------------------------------------------------------
+// 3-D register chains
+// ---------------------------------------------------------------------------
+// As above with a third dimension: a warp's lanes cover 32 x VEC columns of
+// RPY neighbouring rows, the block's warps follow one another along Y, and
+// the block walks Z.  A thread keeps the 2 RZ + 1 newest planes of its rows,
+// and of the RY rows on either side, for each of the T fields; X neighbours
+// come by shuffles, the rows on either side through shared memory: the input
+// planes arrive there by cp.async, DEPTH - 1 steps ahead, and a stage leaves
+// the rows of its new plane there for the next step.  One barrier per plane.
+template <typename T_, int NIN_, int NOUT_, int RZ_, int RY_, int RX_, int NT_, int TEMPORAL_,
+          int LOADER_, int VEC_, int RPY_>
+struct PlaneChainCfg {
+  typedef T_ T;
+  static constexpr int NIN = NIN_, NOUT = NOUT_;
+  static constexpr int RZ = RZ_, RY = RY_, RX = RX_;   // radius of ONE step
+  static constexpr int NT = NT_, TEMPORAL = TEMPORAL_, LOADER = LOADER_, VEC = VEC_, RPY = RPY_;
+  static constexpr int ALIGN = 16 / (int)sizeof(T);
+  static constexpr int W = 2 * RZ + 1;               // planes of a field's window
+  static constexpr int XR = RPY + 2 * RY;            // rows a thread holds
+  static constexpr int EY = NT / 32 * RPY;           // rows of the block
+  static constexpr int PADL = cdiv(TEMPORAL * RX, VEC) * VEC;
+  static constexpr int TX = (32 * VEC - PADL - TEMPORAL * RX) / VEC * VEC;   // columns stored
+  static constexpr int TY = EY - 2 * TEMPORAL * RY;                          // rows stored
+  static constexpr int ROWS = 1, STAGES = 0, NSLOT = 0, HC = RZ, BC = CSD_BC_NONE, BRICK_SHIFT = 0;
+  static constexpr int BOXW = 32 * VEC, BOXH = EY;
+  static constexpr int DEPTH = 4;                    // input planes staged
+  static constexpr int PLANE = EY * BOXW;            // elements of a staged plane
+  // input ring, then two planes per intermediate field
+  static constexpr int SMEM_BYTES = (DEPTH + 2 * (TEMPORAL - 1)) * NIN * PLANE * (int)sizeof(T);
+  static_assert(VEC % ALIGN == 0, "a lane owns whole 16-byte vectors");
+  static_assert(TX > 0 && TY > 0, "the chain consumes the whole tile");
+  static_assert(RPY >= RY, "the rows on either side are the neighbouring warps'");
+  static_assert(NIN == NOUT, "a temporal chain feeds output field f into input field f");
+};
+
+// The planes a stage reads: row DY of the thread's rows and the RY on either
+// side, columns past the lane's own points from the neighbouring lanes.
+template <class C>
+struct PlaneChainView {
+  typedef typename C::T T;
+  const T (*win)[C::W][C::XR][C::VEC];   // [field][plane slot][row][point], registers
+  int oldest;                            // slot of plane -RZ (constant once unrolled)
+  const double* scal;
+  const double* dyn;
+
+  __device__ __forceinline__ double scalar(int k) const { return scal[k]; }
+  __device__ __forceinline__ double dynamic(int k) const { return dyn[k]; }
+
+  template <int F, int DZ, int DY, int LO, int HI>
+  __device__ __forceinline__ Strip<T, LO, HI, C::VEC> strip(int, int, int) const {
+    const T* row = win[F][(oldest + C::RZ + DZ) % C::W][C::RY + DY];
+    Strip<T, LO, HI, C::VEC> s;
+#pragma unroll
+    for (int i = 0; i < C::VEC + HI - LO; ++i) {
+      const int q = fdiv(LO + i, C::VEC);
+      const T v = row[LO + i - q * C::VEC];
+      s.v[i] = q == 0 ? v
+                      : (q < 0 ? __shfl_up_sync(0xffffffffu, v, -q)
+                               : __shfl_down_sync(0xffffffffu, v, q));
+    }
+    return s;
+  }
+};
+
+// One item (see chain_item); gx0, gy0: array column and row of the thread's
+// first point, yb: that row in the block.
+template <class C, class Body, bool MASKED>
+__device__ __forceinline__ void plane_chain_item(const csd_grid& g, int gx0, int gy0, int yb,
+                                                 int z0, int nrows) {
+  typedef typename C::T T;
+  typedef typename VecOf<T>::type Q;
+  constexpr int T_ = C::TEMPORAL, W = C::W, V = C::VEC, RZ = C::RZ, RY = C::RY, R = C::RPY;
+  constexpr int XR = C::XR, D = C::DEPTH, BW = C::BOXW;
+  const int lane = threadIdx.x & 31;
+  const int nz = g.interior[0];
+  const int hx = g.halo[2], xend = hx + g.interior[2];
+  const int hy = g.halo[1], yend = hy + g.interior[1];
+  const int NZ = (int)g.dims[0], NY = (int)g.dims[1], NX = (int)g.dims[2];
+  const long long pitch = g.pitch_z, pitch_y = g.pitch_y;
+  const bool xin = gx0 >= hx && gx0 + V <= xend;
+  const bool vec_store = g.vec_store != 0;
+  bool in[R][V], mine[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const bool yin = gy0 + r >= hy && gy0 + r < yend;
+#pragma unroll
+    for (int e = 0; e < V; ++e) in[r][e] = yin && gx0 + e >= hx && gx0 + e < xend;
+    mine[r] = lane >= C::PADL / V && lane < (C::PADL + C::TX) / V && yin &&
+              yb + r >= T_ * RY && yb + r < C::EY - T_ * RY;
+  }
+  const int n = nrows + 2 * T_ * RZ;               // input planes of the item
+  const int zin = g.halo[0] + z0 - T_ * RZ;        // array plane of input plane 0
+  long long at = (long long)zin * pitch + (long long)gy0 * pitch_y + gx0;   // next request
+  long long to = (long long)(g.halo[0] + z0) * pitch + (long long)gy0 * pitch_y + gx0;
+
+  extern __shared__ __align__(128) unsigned char smem_dyn[];
+  T* ring = reinterpret_cast<T*>(smem_dyn);                 // [slot][field][row][column]
+  T* exch = ring + D * C::NIN * C::PLANE;                   // [stage][parity][field][row][column]
+  // the lane's vectors of staged row r of the block
+  auto vec_load = [&](const T* plane, int r, T (&v)[V]) {
+#pragma unroll
+    for (int e = 0; e < V; e += C::ALIGN)
+      *reinterpret_cast<Q*>(&v[e]) = *reinterpret_cast<const Q*>(plane + r * BW + lane * V + e);
+  };
+  auto request_plane = [&](int j) {
+    const bool plane = j < n && (!MASKED || (zin + j >= 0 && zin + j < NZ));
+#pragma unroll
+    for (int f = 0; f < C::NIN; ++f) {
+      const T* base = reinterpret_cast<const T*>(g.in[f]);
+      constexpr int STEP = C::LOADER == CSD_LOADER_TMA ? C::ALIGN : 1;   // points per copy
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const T* src = base + at + r * pitch_y;
+        const unsigned dst = ptx::smem_addr(ring + ((j % D) * C::NIN + f) * C::PLANE +
+                                            (yb + r) * BW + lane * V);
+#pragma unroll
+        for (int e = 0; e < V; e += STEP) {
+          int have = STEP;   // points of the copy inside the array
+          if (MASKED)
+            have = gx0 + e < 0 || gy0 + r < 0 || gy0 + r >= NY ? 0
+                                                               : min(max(NX - (gx0 + e), 0), STEP);
+          if (!plane) have = 0;
+          const T* from = have > 0 ? src + e : base;
+          if constexpr (STEP > 1)
+            ptx::cp_async_16_partial(dst + e * (int)sizeof(T), from, have * (int)sizeof(T));
+          else
+            ptx::cp_async_zfill<sizeof(T)>(dst + e * (int)sizeof(T), from, have > 0);
+        }
+      }
+    }
+    at += pitch;
+    ptx::cp_async_commit();   // one group per plane, empty past the last
+  };
+
+  T win[T_][C::NIN][W][XR][V];
+#pragma unroll
+  for (int s = 0; s < T_; ++s)
+#pragma unroll
+    for (int f = 0; f < C::NIN; ++f)
+#pragma unroll
+      for (int u = 0; u < W; ++u)
+#pragma unroll
+        for (int r = 0; r < XR; ++r)
+#pragma unroll
+          for (int e = 0; e < V; ++e) win[s][f][u][r][e] = T(0);
+  __syncthreads();   // the previous item's planes have been read
+#pragma unroll 1
+  for (int j = 0; j < D - 1; ++j) request_plane(j);
+
+  // Step j takes in input plane j; stage s computes plane j - (s - 1) - s RZ
+  // of its field, from planes whose rows were exchanged by earlier steps.
+  const int steps = n + T_ - 1;
+#pragma unroll 1
+  for (int j0 = 0; j0 < steps; j0 += W) {
+#pragma unroll
+    for (int u = 0; u < W; ++u) {
+      const int j = j0 + u;
+      ptx::cp_async_wait<D - 2>();
+      __syncthreads();   // input plane j and the rows left by step j - 1 are there
+      request_plane(j + D - 1);   // into the slot of plane j - 1
+#pragma unroll
+      for (int f = 0; f < C::NIN; ++f) {
+        const T* plane = ring + ((j % D) * C::NIN + f) * C::PLANE;
+#pragma unroll
+        for (int r = 0; r < XR; ++r)
+          vec_load(plane, min(max(yb + r - RY, 0), C::EY - 1), win[0][f][u][r]);
+#pragma unroll
+        for (int s = 1; s < T_; ++s) {
+          const T* left = exch + (((s - 1) * 2 + ((j + 1) & 1)) * C::NIN + f) * C::PLANE;
+#pragma unroll
+          for (int r = 0; r < XR; ++r)
+            if (r < RY || r >= RY + R)
+              vec_load(left, min(max(yb + r - RY, 0), C::EY - 1),
+                       win[s < T_ ? s : 0][f][(u + W - 1) % W][r]);
+        }
+      }
+#pragma unroll
+      for (int s = T_; s >= 1; --s) {
+        OutPack<T, C::NOUT, V * R> o;
+        const PlaneChainView<C> view{win[s - 1], s == 1 ? (u + 1) % W : u, g.scalars, g.dyn};
+        Body::template compute<C>(view, 0, 0, 0, o);
+        if (s == T_) {
+          if (j >= 2 * T_ * RZ + T_ - 1 && j < steps) {
+#pragma unroll
+            for (int f = 0; f < C::NOUT; ++f)
+#pragma unroll
+              for (int r = 0; r < R; ++r) {
+                T* out = reinterpret_cast<T*>(g.out[f]) + to + r * pitch_y;
+                if (mine[r]) {
+                  if (vec_store && (!MASKED || xin)) {
+                    store_unit<V>(out, &o.v[f][r * V]);
+                  } else {
+#pragma unroll
+                    for (int e = 0; e < V; ++e)
+                      if (!MASKED || in[r][e]) out[e] = o.v[f][r * V + e];
+                  }
+                }
+              }
+            to += pitch;
+          }
+        } else {
+          // intermediate fields are zero outside the interior
+          const int zr = z0 - T_ * RZ + j - (s - 1) - s * RZ;
+          const bool zi = !MASKED || (unsigned)zr < (unsigned)nz;
+#pragma unroll
+          for (int f = 0; f < C::NOUT; ++f) {
+            T* left = exch + (((s - 1) * 2 + (j & 1)) * C::NIN + f) * C::PLANE;
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+              T w[V];
+#pragma unroll
+              for (int e = 0; e < V; ++e) {
+                w[e] = !MASKED || (zi && in[r][e]) ? o.v[f][r * V + e] : T(0);
+                win[s < T_ ? s : 0][f][u][RY + r][e] = w[e];
+              }
+              if (r < RY || r >= R - RY) store_unit<V>(left + (yb + r) * BW + lane * V, w);
+            }
+          }
+        }
+      }
+    }
+  }
+  ptx::cp_async_wait<0>();
+}
+
+template <class C, class Body, bool BATCHED>
+__device__ __forceinline__ void plane_chain_items(const csd_params& p) {
+  constexpr int T_ = C::TEMPORAL;
+  const int total = BATCHED ? p.total_items : p.g.items;
+  const int yb = (int)(threadIdx.x >> 5) * C::RPY;
+  for (int gitem = blockIdx.x; gitem < total; gitem += gridDim.x) {
+    int item = gitem;
+    const csd_grid& g = BATCHED ? p.grids[batch_grid_of(p, gitem, item)] : p.g;
+    int tx, ty, z0, nrows;
+    csd_item_place(&g, item, &tx, &ty, &z0, &nrows);
+    const int x0 = g.xbase + tx * C::TX - C::PADL;          // array column of the block's first point
+    const int y0 = g.ybase + ty * C::TY - T_ * C::RY;       // ... and row
+    const bool inside = x0 >= g.halo[2] && x0 + 32 * C::VEC <= g.halo[2] + g.interior[2] &&
+                        y0 >= g.halo[1] && y0 + C::EY <= g.halo[1] + g.interior[1] &&
+                        z0 - T_ * C::RZ >= 0 && z0 + nrows + T_ * C::RZ <= g.interior[0];
+    const int gx0 = x0 + (int)(threadIdx.x & 31) * C::VEC;
+    if (inside)
+      plane_chain_item<C, Body, false>(g, gx0, y0 + yb, yb, z0, nrows);
+    else
+      plane_chain_item<C, Body, true>(g, gx0, y0 + yb, yb, z0, nrows);
+  }
+}
+
+template <class C, class Body>
+__device__ __forceinline__ void plane_chain(const csd_params& p) {
+  if (p.grids == nullptr)
+    plane_chain_items<C, Body, false>(p);
+  else
+    plane_chain_items<C, Body, true>(p);
+}
+
+// ---------------------------------------------------------------------------
 // Direct kernels: one step from global memory, rows of any pitch
 // ---------------------------------------------------------------------------
 // Neither tensor copies nor 16-byte vectors reach rows whose pitch is not a

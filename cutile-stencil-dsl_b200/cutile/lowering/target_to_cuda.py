@@ -322,9 +322,6 @@ def emit_body(kernel: KernelOp, vec: int | None = None, suffix: str = "",
     return "\n".join(out)
 
 
-CHAIN_THREADS = 128   # four independent warps per block of a register chain
-
-
 DIRECT_THREADS = 256
 
 
@@ -477,7 +474,8 @@ def engine_params(kernel: KernelOp) -> dict:
         "NDYN": kernel.dyn_count.data if kernel.dyn_count is not None else 0,
         "REDUCE": kernel.reduce_max.data if kernel.reduce_max is not None else 0,
         "BRICK": _brick_code(kernel, ndim),
-        "RPY": int(hints.get("rpy", 1)),
+        "RPY": int(hints.get("chain_rows", 0) or hints.get("rpy", 1)),
+        "CHAIN_WARPS": int(hints.get("chain_warps", 4)),   # warps per block of a register chain
         "OCCUPANCY": int(hints.get("occupancy", 0)),   # a caller's blocks per SM (0: none)
         # points per lane of a register chain (0: the ring engine)
         "CHAIN": int(hints.get("register_chain", 0)),
@@ -548,9 +546,14 @@ def emit_cuda(module: ModuleOp, preamble: bool = True) -> str:
                    f"{p['ROWS']}, {p['TY']}, {p['TX']}, {p['NT']}, {p['STAGES']}, {p['TEMPORAL']}, "
                    f"{loader}, {p['BC']}, {p['REDUCE']}, {p['BRICK']}, {p['RPY']}, {p['VEC']}>")
             if p["CHAIN"]:
-                entry, nt, minb = "register_chain", CHAIN_THREADS, 1
+                entry, nt, minb = "register_chain", 32 * p["CHAIN_WARPS"], 1
                 cfg = (f"csd::ChainCfg<{p['T']}, {p['NIN']}, {p['NOUT']}, {p['RZ']}, {p['RX']}, "
                        f"{nt}, {p['TEMPORAL']}, {loader}, {p['VEC']}>")
+                if p["ndim"] == 3:
+                    entry = "plane_chain"
+                    cfg = (f"csd::PlaneChainCfg<{p['T']}, {p['NIN']}, {p['NOUT']}, {p['RZ']}, "
+                           f"{p['RY']}, {p['RX']}, {nt}, {p['TEMPORAL']}, {loader}, {p['VEC']}, "
+                           f"{p['RPY']}>")
             parts.append(f"typedef {cfg} Cfg_{name}_{suffix};")
             parts.append(f'extern "C" __global__ void __launch_bounds__({nt}, {minb})')
             parts.append(f"{name}_{suffix}(const __grid_constant__ csd_params p) {{")

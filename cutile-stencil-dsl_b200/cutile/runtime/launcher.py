@@ -490,10 +490,23 @@ def chain_tile_2d(dtype_bytes: int, T: int) -> dict:
     return dict(rows=4, tile_x=128, threads=256)
 
 
-def register_chain_points(radius, dtype_bytes: int, num_inputs: int, T: int,
-                          body_ops: int) -> int:
-    """Points per lane of the register chain (engine.cuh ``ChainCfg``) for a
-    chain of T steps, or 0 where the shared-memory rings keep it.
+def _side_planes(ir) -> int:
+    """Planes of the rows beside a thread's own that a 3-D register chain
+    holds: from the leading plane to the last one the body reads off centre."""
+    from cutile.dialects.stencil import AccessOp
+
+    offs = [tuple(op.offset) for op in ir.walk() if isinstance(op, AccessOp)]
+    if not offs or len(offs[0]) != 3:
+        return 0
+    lead = max(o[0] for o in offs)
+    return max((lead - o[0] + 1 for o in offs if o[1] != 0), default=0)
+
+
+def register_chain_plan(radius, dtype_bytes: int, num_inputs: int, T: int, body_ops: int,
+                        side_planes: int = 0) -> dict:
+    """Hints of the register chain (engine.cuh ``ChainCfg``,
+    ``PlaneChainCfg``) for a chain of T steps: points per lane, and in 3-D rows
+    per thread and warps per block; {} where the shared-memory rings keep it.
 
     1-D and 2-D chains whose windows fit the registers take it.  Measured on
     B200 per launch, rings -> registers: heat 1024^2 FP64 T=5 103 -> 10.9 us,
@@ -501,10 +514,29 @@ def register_chain_points(radius, dtype_bytes: int, num_inputs: int, T: int,
     and 275 -> 73; radius 2 FP64 T=4 80 -> 25 and 315 -> 170; heat1d 2^22 T=8
     FP64 123 -> 18, FP32 68 -> 10.  The one loss seen is a radius-2 FP32 chain
     of three or four steps on a grid too small to fill the chip (200 x 300:
-    8.5 -> 9.9 and 12.2 -> 16.0 us; 1024^2: 28 -> 15 and 51 -> 28)."""
+    8.5 -> 9.9 and 12.2 -> 16.0 us; 1024^2: 28 -> 15 and 51 -> 28).
+
+    3-D chains take it as far as their windows fit: two rows per thread and
+    sixteen warps while a block of them keeps 128 registers each, else three
+    rows and eight warps.  7-point 384^3 per launch, rings -> registers: FP64
+    T=2 329 -> 212 us, T=4 982 -> 487; FP32 T=2 186 -> 148, T=4
+    559 -> 423 (one row per thread 327 and 202 for T=2, three rows and
+    eight warps 266 and 187).  Chains of several fields keep the rings (FP32
+    Kahan T=2: rings 308 us, registers 345)."""
     ndim = len(radius)
-    if ndim > 2:
-        return 0
+    if ndim == 3:
+        rz, ry, rx = radius
+        vec = 16 // dtype_bytes
+        pad = -(-T * rx // vec) * vec
+        for rows, warps, budget in ((2, 16, 84), (3, 8, 210)):
+            # 32-bit registers of the T windows: own rows, rows on either side
+            words = T * (rows * (2 * rz + 1) + 2 * ry * side_planes) * 4
+            # at least half of the block's rows and columns are stored
+            if (num_inputs == 1 and words <= budget and ry <= rows and 4 * T * ry <= rows * warps
+                    and 2 * (32 * vec - pad - T * rx) >= 32 * vec
+                    and T * (2 * rz + 1) * rows * body_ops <= 4000):
+                return {"register_chain": vec, "chain_rows": rows, "chain_warps": warps}
+        return {}
     rz, rx = (radius[0] if ndim == 2 else 0), radius[-1]
     # one 16-byte vector per lane; two in 1-D, where no rows are kept (FP32
     # 2^22: 14.8 us with one, 10.1 with two, 10.2 with four)
@@ -514,10 +546,10 @@ def register_chain_points(radius, dtype_bytes: int, num_inputs: int, T: int,
     # unrolled code (2 rz + 1 copies of every stage's body)
     window = T * num_inputs * (2 * rz + 1) * vec * dtype_bytes // 4
     if window > 192 or T * (2 * rz + 1) * body_ops > 3000:
-        return 0
+        return {}
     # the strip's stored columns: at least half of the 32 lanes' points
     pad = -(-T * rx // vec) * vec
-    return vec if 2 * (32 * vec - pad - T * rx) >= 32 * vec else 0
+    return {"register_chain": vec} if 2 * (32 * vec - pad - T * rx) >= 32 * vec else {}
 
 
 def _rpy_keeps_registers(stencil_fn, plan, stencil_halo, halo_widths, dtype, dtype_bytes,
@@ -669,12 +701,12 @@ def compile(stencil_fn, domain: tuple[int, ...] | None = None, hw=None,
         hints["occupancy"] = occupancy
     if T > 1 and layout != "bricked":
         if kernel_hints and "register_chain" in kernel_hints:
-            hints["register_chain"] = int(kernel_hints["register_chain"])
+            for k in ("register_chain", "chain_rows", "chain_warps"):
+                if k in kernel_hints:
+                    hints[k] = int(kernel_hints[k])
         elif tile_sizes is None and not kernel_hints and occupancy is None:
-            points = register_chain_points(stencil_halo, dtype_bytes, num_inputs, T,
-                                           analysis.get("body_ops", 0))
-            if points:
-                hints["register_chain"] = points
+            hints.update(register_chain_plan(stencil_halo, dtype_bytes, num_inputs, T,
+                                             analysis.get("body_ops", 0), _side_planes(clone)))
 
     boundary_spec = None
     if getattr(stencil_fn, "_boundary", None) is not None:

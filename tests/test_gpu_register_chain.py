@@ -103,3 +103,83 @@ def test_batched_chain_equals_single_launches():
     torch.cuda.synchronize()
     for a, b in zip(outs, alone):
         assert torch.equal(a, b)
+
+
+def skewed(u, i, j, k):
+    return (0.5 * u[i, j, k] + 0.25 * u[i + 1, j - 1, k] - 0.125 * u[i, j + 1, k - 1]
+            + 0.0625 * u[i - 1, j, k + 1])
+
+
+@pytest.mark.parametrize("align_halo", [True, False])
+@pytest.mark.parametrize("fn,dtype,T", [
+    (D.lap7, "float64", 2), (D.lap7, "float32", 3), (D.lap7, "float64", 4), (D.box27, "float64", 2),
+    (skewed, "float32", 2)])
+def test_3d_tile_edges(fn, dtype, T, align_halo):
+    """Columns and rows around whole tiles, one plane to several items of
+    planes, halos that are not zero, aligned and per-element copies."""
+    import cutile
+    from cutile import stencil
+
+    r = cutile.compile(stencil(ndim=3, dtype=dtype)(fn), temporal_steps=T, align_halo=align_halo)
+    assert r.temporal_steps == T and r.kernel_hints["chain_rows"] > 0
+    d = r.load_module().program().kernel().desc
+    tx, ty = d["tile_x"], d["tile_y"]
+    rng = np.random.default_rng(T)
+    for nz, ny, nx in ((1, 1, 1), (2, ty - 1, tx - 1), (9, ty, tx), (5, ty + 1, tx + 1),
+                       (13, 2 * ty + 3, 2 * tx + 5)):
+        shape = tuple(s + 2 * h for s, h in zip((nz, ny, nx), r.halo_widths))
+        u = rng.standard_normal(shape).astype(dtype)
+        want = O.temporal_launch(u, np.full(shape, np.nan, dtype=dtype), fn, 3, r.halo_widths, T)
+        for zchunk in (0, 4):
+            got = _launch(r, u, zchunk=zchunk)
+            assert np.array_equal(got, want, equal_nan=True), (shape, zchunk)
+
+
+def test_3d_kahan_chain_keeps_both_fields():
+    """Two fields (u and its compensation) chained in three dimensions equal
+    separate single steps through zero-halo buffers."""
+    import torch
+
+    import cutile
+    from cutile import stencil
+
+    fn = stencil(ndim=3, dtype="float32")(D.lap7)
+    r = cutile.compile(fn, precision="fp32_kahan", temporal_steps=2, kernel_hints={
+        "register_chain": 4, "chain_rows": 3, "chain_warps": 8})
+    r1 = cutile.compile(fn, precision="fp32_kahan", temporal_blocking=False)
+    shape = tuple(s + 2 * h for s, h in zip((9, 40, 150), r.halo_widths))
+    inner = tuple(slice(h, s - h) for h, s in zip(r.halo_widths, shape))
+    a = [torch.zeros(shape, device="cuda") for _ in range(2)]
+    a[0][inner] = torch.randn(a[0][inner].shape, device="cuda")
+    a[1][inner] = 1e-8 * torch.randn(a[0][inner].shape, device="cuda")
+    got = [torch.zeros_like(x) for x in a]
+    r.load_module().launch_lap7(*a, *got)
+    for _ in range(2):
+        b = [torch.zeros_like(x) for x in a]
+        r1.load_module().launch_lap7(*a, *b)
+        a = b
+    assert torch.equal(got[0], a[0]) and torch.equal(got[1], a[1])
+
+
+def test_3d_batched_chain_equals_single_launches():
+    import torch
+
+    import cutile
+    from cutile import stencil
+    from cutile.runtime.rk_runtime import BatchLaunch
+
+    r = cutile.compile(stencil(ndim=3)(D.lap7), temporal_steps=2)
+    prog = r.load_module().program()
+    ins, outs, alone = [], [], []
+    for shape in ((9, 40, 70), (30, 5, 33), (3, 29, 61)):
+        shape = tuple(s + 2 * h for s, h in zip(shape, r.halo_widths))
+        wide = torch.randn(shape[:2] + (-(-shape[2] // 16) * 16,), dtype=torch.float64, device="cuda")
+        ins.append(wide[..., :shape[2]])
+        outs.append(torch.zeros_like(wide)[..., :shape[2]])
+        alone.append(torch.zeros_like(wide)[..., :shape[2]])
+        prog.launch([ins[-1]], [alone[-1]])
+    per = [{"inputs": [i], "outputs": [o]} for i, o in zip(ins, outs)]
+    BatchLaunch(prog.kernel(), per, r.halo_widths, zchunk=7).launch()
+    torch.cuda.synchronize()
+    for a, b in zip(outs, alone):
+        assert torch.equal(a, b)
