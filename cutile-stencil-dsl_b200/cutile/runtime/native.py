@@ -484,6 +484,33 @@ def grid_build(kernel: NativeKernel, inputs, outputs, halo, dest, **kw) -> tuple
     return items.value, loader.value
 
 
+def grid_build_rotations(kernel: NativeKernel, bufs, nstate: int, halo, dest: int, **kw) -> int:
+    """Descriptors of one grid at every phase of its buffer rotation, one
+    after the other at host address ``dest``: at phase p the kernel reads
+    ``bufs[p], bufs[p - 1], ...`` (``nstate`` of them) and writes
+    ``bufs[p + 1]``.  Returns the grid's work items (the same at every phase)."""
+    lib = library()
+    P = len(bufs)
+    f = [field_of(t, True) for t in bufs]
+    o = make_opts(halo, **kw)
+    items, loader = ctypes.c_int(), ctypes.c_int()
+    gsz = grid_size()
+    for p in range(P):
+        fin = (Field * nstate)(*[f[(p - k) % P] for k in range(nstate)])
+        check(lib.csd_grid_build(kernel.handle, fin, nstate, ctypes.byref(f[(p + 1) % P]), 1,
+                                 ctypes.byref(o), dest + p * gsz, ctypes.byref(items),
+                                 ctypes.byref(loader)))
+    return items.value
+
+
+def batch_opts(loader: int, grid_index_ptr: int):
+    """Reusable csd_launch_batch options (kept alive by the reference)."""
+    o = LaunchOpts()
+    o.loader = loader
+    o.grid_index = grid_index_ptr
+    return ctypes.byref(o)
+
+
 def launch_batch(kernel: NativeKernel, grids_ptr: int, item_start_ptr: int, ngrids: int,
                  total_items: int, stream=None, grid: int = 0, timeout_ns: int = 0,
                  loader: int = 0, grid_index_ptr: int | None = None) -> None:
@@ -611,6 +638,6 @@ def error_word(reset: bool = True) -> int:
 
 __all__ = ["library", "check", "compile_source", "NativeModule", "NativeKernel", "launch",
            "apply_boundary", "error_word", "error_status", "CSD_ETIMEOUT", "CSD_ERR_TIMEOUT", "CsdError", "field_of", "default_cache_dir",
-           "make_opts", "LaunchPlans", "grid_size", "grid_build", "launch_batch", "bricked_shape",
+           "make_opts", "LaunchPlans", "grid_build_rotations", "batch_opts", "grid_size", "grid_build", "launch_batch", "bricked_shape",
            "to_bricks", "from_bricks", "bricked_field", "launch_fields",
            "GridHead", "plan_items", "NVCC_OPTIONS", "find_nvcc", "aot_compile", "read_image", "CSD_LOADER_TMA", "CSD_LOADER_LDG", "BC_MODES"]
