@@ -297,6 +297,36 @@ __device__ __forceinline__ double sqrt_rn(double x) {
   return z ? x : r;
 }
 
+// FP64 division by a value that many quotients share (a grid spacing, a
+// constant).  With r = RN(1/y), a quotient estimate q within one ulp of x/y and
+// the exact remainder x - q y (one fused multiply-add), RN(q + r (x - q y)) is
+// the correctly rounded quotient (P. Markstein, IBM J. Res. Dev. 34, 1990); the
+// first such step brings q = RN(x r) within one ulp, the second rounds.  That
+// holds while nothing over- or underflows: with x and y within 2^+-480 of 1
+// the quotient is normal and so is the remainder, a multiple of at least
+// 2^-107 |x|.  A zero x takes x r, a zero of the right sign; the rest goes to
+// div_rn.
+struct Divisor {
+  double y, r;   // the divisor and its correctly rounded reciprocal
+  bool ok;       // y in the range above
+};
+// |x| in [2^-480, 2^480)
+__device__ __forceinline__ bool quotient_safe(double x) {
+  return ((unsigned)__double2hiint(x) & 0x7fffffffu) - (543u << 20) < (960u << 20);
+}
+__device__ __forceinline__ Divisor divisor(double y) {
+  return {y, __drcp_rn(y), quotient_safe(y)};
+}
+__device__ __forceinline__ double div_by(double x, const Divisor& d) {
+  const double q0 = __dmul_rn(x, d.r);
+  const double q1 = __fma_rn(__fma_rn(-q0, d.y, x), d.r, q0);
+  const double q2 = __fma_rn(__fma_rn(-q1, d.y, x), d.r, q1);
+  const bool in = quotient_safe(x);
+  double q = in ? q2 : q0;
+  if (!((in || x == 0.0) && d.ok)) q = div_rn(x, d.y);
+  return q;
+}
+
 // Element offset of array cell (z, y, x) (internal 3-D view): pitched rows,
 // or bricks of B^ndim elements (brick-major, row-major inside a brick).
 template <class C>
