@@ -90,17 +90,18 @@ struct Cfg {
   static constexpr int ALIGN = 16 / (int)sizeof(T);
   // points per unit along X: one 16-byte vector by default; a wider unit
   // (several vectors) reads each staged row group with fewer strips per
-  // point, for single-step flat kernels with one row per thread
+  // point, a narrower one (a power-of-two part of a vector) has less code and
+  // fewer registers; both for single-step flat kernels, one row per thread
   static constexpr int VEC = VEC_ > 0 ? VEC_ : ALIGN;
-  static_assert(VEC % ALIGN == 0 &&
+  static_assert((VEC % ALIGN == 0 || ALIGN % VEC == 0) &&
                     (VEC == ALIGN || (TEMPORAL_ == 1 && BRICK_ == 0 && RPY_ == 1)),
-                "units wider than one vector: single-step flat kernels, one row per thread");
+                "other units than one vector: single-step flat kernels, one row per thread");
   static constexpr int HC = RZ > 0 ? cdiv(RZ, ROWS) : 0;  // halo chunks per side, per step
   // Column layout shared by every buffer: smem column c <-> x = X0 - PADL + c.
   // bricked TMA rows: whole bricks, each row 128-byte aligned (TMA destination)
   static constexpr int BALIGN = imax(BRICK_B, 128 / (int)sizeof(T));
   static constexpr int PADL = BTMA ? align_up(RX, BRICK_B)
-                            : TEMPORAL == 1 ? align_up(RX, VEC)
+                            : TEMPORAL == 1 ? align_up(RX, imax(VEC, ALIGN))
                                             : align_up(TEMPORAL * RX + 2 * ALIGN - 2, ALIGN);
   static constexpr int BOXW = BTMA ? align_up(PADL + TX + RX, BALIGN)
                             : TEMPORAL == 1 ? align_up(PADL + TX + RX, ALIGN)
@@ -168,13 +169,29 @@ struct Strip {
   T v[VEC + HI - LO];
 };
 
-template <typename T, int LO, int HI, int VEC, int ALIGN>
+// the vector of N elements
+template <typename T, int N>
+struct VecN {
+  typedef typename VecOf<T>::type type;
+};
+template <typename T>
+struct VecN<T, 1> {
+  typedef T type;
+};
+template <>
+struct VecN<float, 2> {
+  typedef float2 type;
+};
+
+template <typename T, int LO, int HI, int VEC, int ALIGN_>
 __device__ __forceinline__ Strip<T, LO, HI, VEC> load_strip(const T* row, int x) {
-  // row: smem row base; x: column of the unit's first point (multiple of ALIGN)
+  // row: smem row base; x: column of the unit's first point (multiple of
+  // ALIGN: the unit, or 16 bytes of a longer one)
+  constexpr int ALIGN = VEC < ALIGN_ ? VEC : ALIGN_;
   constexpr int A0 = fdiv(LO, ALIGN) * ALIGN;             // aligned start offset
   constexpr int A1 = align_up(VEC + HI, ALIGN);            // aligned end offset (exclusive)
   constexpr int NV = (A1 - A0) / ALIGN;
-  typedef typename VecOf<T>::type V;
+  typedef typename VecN<T, ALIGN>::type V;
   T buf[NV * ALIGN];
   const V* src = reinterpret_cast<const V*>(row + x + A0);
 #pragma unroll
@@ -233,8 +250,16 @@ __device__ __forceinline__ void store_vec(float* p, const float* v) {
 template <int VEC, typename T>
 __device__ __forceinline__ void store_unit(T* p, const T* v) {
   constexpr int A = 16 / (int)sizeof(T);
+  if constexpr (VEC >= A) {
 #pragma unroll
-  for (int i = 0; i < VEC; i += A) store_vec(p + i, v + i);
+    for (int i = 0; i < VEC; i += A) store_vec(p + i, v + i);
+  } else {
+    typedef typename VecN<T, VEC>::type V;
+    V t;
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) reinterpret_cast<T*>(&t)[i] = v[i];
+    *reinterpret_cast<V*>(p) = t;
+  }
 }
 
 // Fused boundary fill: map an out-of-interior index of one dim to the

@@ -286,9 +286,10 @@ def fit_plan(plan: EnginePlan, radius: tuple[int, ...], dtype_bytes: int,
     r3 = radius3(plan.ndim, radius)
     if plan.rpy != 1 and (plan.ndim != 3 or plan.temporal != 1 or plan.rpy < 1):
         raise ValueError("rows per thread > 1 needs a 3-D single-step stencil")
-    if plan.vec != 16 // dtype_bytes and (plan.vec % (16 // dtype_bytes) or plan.vec <= 0
-                                          or plan.temporal != 1 or plan.rpy != 1):
-        raise ValueError(f"a {plan.vec}-point unit needs a multiple of {16 // dtype_bytes} points, "
+    full = 16 // dtype_bytes   # points of a 16-byte vector
+    if plan.vec != full and (plan.vec <= 0 or (plan.vec % full and full % plan.vec)
+                             or plan.temporal != 1 or plan.rpy != 1):
+        raise ValueError(f"a {plan.vec}-point unit needs a multiple or a divisor of {full} points, "
                          "one step and one row per thread")
     for _ in range(64):
         g = engine_geometry(plan, r3, dtype_bytes, num_inputs, periodic)

@@ -960,10 +960,14 @@ def build_variants(stencil_fn, variants: dict, *, dtype: str | None = None,
         plan = default_engine_plan(len(stencil_halo), num_loads, dtype_bytes, stencil_halo,
                                    n_fields + extra_in, _yields(ir))
         if len(stencil_halo) == 2 and tile_sizes is None and analysis.get("body_ops", 0) > 120:
-            # long 2-D flux bodies (issue-bound): 64-wide chunks; measured on
-            # the 256-grid shallow-water RK2 batch, 6.82 ms per step against
-            # 7.42 for 128-wide (4 instead of 2 blocks per SM)
-            plan = replace(plan, tile_x=64)
+            # long 2-D flux bodies: what holds them back is latency and the
+            # instruction cache (a unit of four FP32 points is 30 KB of code at
+            # 16 warps per SM), so 8 x 32 chunks, two points per unit and the
+            # registers capped for 24 (FP64 16) warps.  20 shallow-water grids,
+            # 10 RK2 steps: FP32 5.10 -> 4.67 ms (two points in 8 x 64 chunks
+            # 5.36, one 5.75; 4 x 64 chunks 4.74), FP64 10.5 -> 9.7
+            plan = replace(plan, tile_x=32, threads=128, vec=2,
+                           occupancy=6 if dtype_bytes == 4 else 4)
         bmode = opts.pop("boundary_mode", "none")
         plan = fit_plan(_plan_from(tile_sizes, kernel_hints, len(stencil_halo), plan),
                         stencil_halo, dtype_bytes, n_fields + extra_in,
