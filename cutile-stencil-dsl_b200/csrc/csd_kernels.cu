@@ -285,60 +285,89 @@ extern "C" int csd_from_bricks(const void* bricked, int brick, const csd_field* 
 // FP64 reductions over the interior of a field (mass, energy, residual, max)
 //
 // Deterministic: interior rows are cut into segments of RED_SEG elements, and
-// pass 1 gives CTA b the segments [b*S/G, (b+1)*S/G), its warps taking them in
-// turn.  A lane adds its elements in RED_ILP independent FP64 sums in a fixed
-// order, and a fixed-shape tree reduces lanes and warps into partials[b].
-// Pass 2 (one CTA) reduces partials[0..G) the same way.  The result depends on
-// G, never on scheduling.  Bound by HBM: RED_ILP loads per lane and 16 warps
-// per CTA keep enough of them in flight with two CTAs per SM (sum of a 300 x
-// 320 x 340 FP64 interior, 261 MB: 56 us, the difference of two 100; with a
-// row at a time per CTA of 256 threads 388 and 449; a 1-D
-// row, formerly one CTA's, 2^24 FP64: 10.9 ms -> 34 us).
+// pass 1 gives CTA c of C the segments [c*S/C, (c+1)*S/C), its warps taking
+// them in turn.  A lane adds its elements in RED_ACC independent sums in a
+// fixed order, and a fixed-shape tree combines lanes and warps.  Every sum
+// carries the rounding errors of its additions (Knuth's two-sum) beside it, so
+// the result is the exact sum of the FP64 terms but for its last rounding, in
+// nearly all cases; a CTA hands both words on in two of the `nblocks` partials
+// (C = nblocks / 2; a single CTA rounds into one).  Pass 2 (one CTA) combines
+// them the same way.  The result depends on nblocks, never on scheduling.
+// Bound by HBM: RED_ILP loads per lane and 32 warps per SM keep enough of them
+// in flight, and the seven additions per element stay behind them (sum of a
+// 300 x 320 x 340 FP64 interior, 261 MB: 60 us, the difference of two
+// 99; with a row at a time per CTA of 256 threads 388 and 449; a 1-D row,
+// formerly one CTA's, 2^24 FP64: 10.9 ms -> 36 us).
 // ---------------------------------------------------------------------------
 namespace {
 
-constexpr int RED_THREADS = 512, RED_THREADS2 = 256;   // pass 1, pass 2
-constexpr int RED_ILP = 8;
+constexpr int RED_THREADS = 1024, RED_THREADS2 = 256;   // pass 1, pass 2
+constexpr int RED_ILP = 8, RED_ACC = 4;   // loads in flight, sums per lane
 constexpr int RED_SEG = 1024;   // elements of a row segment
 
 template <int OP>
-__device__ __forceinline__ double red_combine(double a, double b) {
-  if (OP == CSD_RED_MAXABS || OP == CSD_RED_DIFF_MAXABS) return (a != a || a > b) ? a : b;
-  return a + b;
+constexpr bool kRedMax = OP == CSD_RED_MAXABS || OP == CSD_RED_DIFF_MAXABS;
+
+// A sum and the rounding errors made in it (maxima: the value alone).
+struct RedSum {
+  double v, err;
+};
+
+template <int OP>
+__device__ __forceinline__ RedSum red_add(RedSum a, double b) {
+  if (kRedMax<OP>) return {(a.v != a.v || a.v > b) ? a.v : b, 0.0};
+  const double s = __dadd_rn(a.v, b);
+  const double t = __dsub_rn(s, a.v);
+  return {s, __dadd_rn(a.err, __dadd_rn(__dsub_rn(a.v, __dsub_rn(s, t)), __dsub_rn(b, t)))};
+}
+template <int OP>
+__device__ __forceinline__ RedSum red_combine(RedSum a, RedSum b) {
+  RedSum s = red_add<OP>(a, b.v);
+  if (!kRedMax<OP>) s.err = __dadd_rn(s.err, b.err);
+  return s;
+}
+// The sum with its errors added back; an infinity or NaN (whose errors mean
+// nothing) as it is.
+template <int OP>
+__device__ __forceinline__ double red_value_of(RedSum a) {
+  return kRedMax<OP> || !isfinite(a.v) ? a.v : __dadd_rn(a.v, a.err);
 }
 
 template <int OP, int THREADS>
-__device__ __forceinline__ double red_block(double v, double* sh) {
+__device__ __forceinline__ RedSum red_block(RedSum v, RedSum* sh) {
   // fixed-shape tree: warp shuffles, then the warp totals in order
-  for (int o = 16; o > 0; o >>= 1) v = red_combine<OP>(v, __shfl_down_sync(0xffffffffu, v, o));
+  for (int o = 16; o > 0; o >>= 1) {
+    const RedSum w = {__shfl_down_sync(0xffffffffu, v.v, o), __shfl_down_sync(0xffffffffu, v.err, o)};
+    v = red_combine<OP>(v, w);
+  }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (lane == 0) sh[warp] = v;
   __syncthreads();
-  double t = 0.0;
+  RedSum t = {0.0, 0.0};
   if (threadIdx.x == 0) {
     t = sh[0];
     for (int w = 1; w < THREADS / 32; ++w) t = red_combine<OP>(t, sh[w]);
   }
-  __syncthreads();
   return t;
 }
 
-// The reduced value of one element.
+// The reduced term of one element.
 template <int OP>
-__device__ __forceinline__ double red_value(double va, double vb) {
+__device__ __forceinline__ double red_term(double va, double vb) {
   if (OP == CSD_RED_SUM) return va;
-  if (OP == CSD_RED_SUMSQ) return va * va;
+  if (OP == CSD_RED_SUMSQ) return __dmul_rn(va, va);
   if (OP == CSD_RED_MAXABS) return fabs(va);
-  const double d = va - vb;
-  return OP == CSD_RED_DIFF_SUMSQ ? d * d : fabs(d);
+  const double d = __dsub_rn(va, vb);
+  return OP == CSD_RED_DIFF_SUMSQ ? __dmul_rn(d, d) : fabs(d);
 }
 
 template <typename T, int OP>
-__global__ void __launch_bounds__(RED_THREADS, 2) reduce_pass1(const T* a, const T* b,
+__global__ void __launch_bounds__(RED_THREADS, 1) reduce_pass1(const T* a, const T* b,
                                                                long long d0, long long d1,
                                                                long long d2, int h0, int h1,
-                                                               int h2, double* partials) {
-  __shared__ double sh[RED_THREADS / 32];
+                                                               int h2, double* partials,
+                                                               int pairs) {
+  __shared__ RedSum sh[RED_THREADS / 32];
   constexpr bool kDiff = OP == CSD_RED_DIFF_SUMSQ || OP == CSD_RED_DIFF_MAXABS;
   const long long ny = d1 - 2 * h1, nx = d2 - 2 * h2;
   const long long nseg = (nx + RED_SEG - 1) / RED_SEG;
@@ -350,9 +379,9 @@ __global__ void __launch_bounds__(RED_THREADS, 2) reduce_pass1(const T* a, const
   long long i = s0 + (threadIdx.x >> 5);
   long long seg = i % nseg, z = i / nseg / ny, y = i / nseg % ny;
   const long long dseg = NW % nseg, dz = NW / nseg / ny, dy = NW / nseg % ny;
-  double acc[RED_ILP];
+  RedSum acc[RED_ACC];
 #pragma unroll
-  for (int k = 0; k < RED_ILP; ++k) acc[k] = 0.0;
+  for (int k = 0; k < RED_ACC; ++k) acc[k] = {0.0, 0.0};
   for (; i < s1; i += NW) {
     const long long base = ((z + h0) * d1 + y + h1) * d2 + h2 + seg * RED_SEG;
     const int n = (int)min((long long)RED_SEG, nx - seg * RED_SEG);
@@ -360,18 +389,23 @@ __global__ void __launch_bounds__(RED_THREADS, 2) reduce_pass1(const T* a, const
     const T* pb = kDiff ? b + base : nullptr;
     int x = lane;
     for (; x + 32 * (RED_ILP - 1) < n; x += 32 * RED_ILP) {
-      double v[RED_ILP];
+      T va[RED_ILP], vb[RED_ILP];
+#pragma unroll
+      for (int k = 0; k < RED_ILP; ++k) {
+        va[k] = pa[x + 32 * k];
+        vb[k] = kDiff ? pb[x + 32 * k] : T(0);
+      }
 #pragma unroll
       for (int k = 0; k < RED_ILP; ++k)
-        v[k] = red_value<OP>((double)pa[x + 32 * k], kDiff ? (double)pb[x + 32 * k] : 0.0);
-#pragma unroll
-      for (int k = 0; k < RED_ILP; ++k) acc[k] = red_combine<OP>(acc[k], v[k]);
+        acc[k % RED_ACC] =
+            red_add<OP>(acc[k % RED_ACC], red_term<OP>((double)va[k], (double)vb[k]));
     }
 #pragma unroll
     for (int k = 0; k < RED_ILP; ++k)
       if (x + 32 * k < n)
-        acc[k] = red_combine<OP>(acc[k], red_value<OP>((double)pa[x + 32 * k],
-                                                       kDiff ? (double)pb[x + 32 * k] : 0.0));
+        acc[k % RED_ACC] = red_add<OP>(
+            acc[k % RED_ACC],
+            red_term<OP>((double)pa[x + 32 * k], kDiff ? (double)pb[x + 32 * k] : 0.0));
     seg += dseg;
     y += dy;
     z += dz;
@@ -385,21 +419,31 @@ __global__ void __launch_bounds__(RED_THREADS, 2) reduce_pass1(const T* a, const
     }
   }
 #pragma unroll
-  for (int w = RED_ILP / 2; w > 0; w >>= 1)
+  for (int w = RED_ACC / 2; w > 0; w >>= 1)
 #pragma unroll
     for (int k = 0; k < w; ++k) acc[k] = red_combine<OP>(acc[k], acc[k + w]);
-  const double t = red_block<OP, RED_THREADS>(acc[0], sh);
-  if (threadIdx.x == 0) partials[blockIdx.x] = t;
+  const RedSum t = red_block<OP, RED_THREADS>(acc[0], sh);
+  if (threadIdx.x == 0) {
+    if (pairs) {
+      partials[2 * blockIdx.x] = t.v;
+      partials[2 * blockIdx.x + 1] = t.err;
+    } else {
+      partials[blockIdx.x] = red_value_of<OP>(t);
+    }
+  }
 }
 
 template <int OP>
 __global__ void __launch_bounds__(RED_THREADS2) reduce_pass2(const double* partials, int n,
-                                                             double* result) {
-  __shared__ double sh[RED_THREADS2 / 32];
-  double acc = 0.0;
-  for (int i = threadIdx.x; i < n; i += RED_THREADS2) acc = red_combine<OP>(acc, partials[i]);
-  const double t = red_block<OP, RED_THREADS2>(acc, sh);
-  if (threadIdx.x == 0) *result = t;
+                                                             int pairs, double* result) {
+  __shared__ RedSum sh[RED_THREADS2 / 32];
+  RedSum acc = {0.0, 0.0};
+  for (int i = threadIdx.x; i < n; i += RED_THREADS2) {
+    const RedSum p = {pairs ? partials[2 * i] : partials[i], pairs ? partials[2 * i + 1] : 0.0};
+    acc = red_combine<OP>(acc, p);
+  }
+  const RedSum t = red_block<OP, RED_THREADS2>(acc, sh);
+  if (threadIdx.x == 0) *result = red_value_of<OP>(t);
 }
 
 template <typename T, int OP>
@@ -407,9 +451,10 @@ int reduce_t(const csd_field* a, const csd_field* b, const long long d[3], const
              double* partials, int nblocks, double* result, cudaStream_t s) {
   const T* pa = reinterpret_cast<const T*>(a->ptr);
   const T* pb = b ? reinterpret_cast<const T*>(b->ptr) : nullptr;
-  reduce_pass1<T, OP><<<nblocks, RED_THREADS, 0, s>>>(pa, pb, d[0], d[1], d[2], h[0], h[1], h[2],
-                                                      partials);
-  reduce_pass2<OP><<<1, RED_THREADS2, 0, s>>>(partials, nblocks, result);
+  const int pairs = nblocks >= 2, ctas = pairs ? nblocks / 2 : nblocks;
+  reduce_pass1<T, OP><<<ctas, RED_THREADS, 0, s>>>(pa, pb, d[0], d[1], d[2], h[0], h[1], h[2],
+                                                   partials, pairs);
+  reduce_pass2<OP><<<1, RED_THREADS2, 0, s>>>(partials, ctas, pairs, result);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? CSD_OK : csd_internal_fail(CSD_ELAUNCH, cudaGetErrorString(e));
 }

@@ -1,8 +1,8 @@
 """FP64 global reductions on the device: mass, energy, residual, max.
 
-Fields may be float32 or float64; accumulation is FP64 in a fixed order
-(``csd_reduce``: one partial per block, then one block over the partials),
-so a result depends on the number of blocks only, never on scheduling --
+Fields may be float32 or float64; accumulation is FP64 in a fixed order with
+the rounding errors carried along (``csd_reduce``: sums per block, then one
+block over them), so a result depends on the number of blocks only, never on scheduling --
 repeated runs and co-scheduled work give identical bits.  Results stay on
 the device as 0-d float64 tensors (read them with ``.item()`` when needed).
 """

@@ -180,9 +180,10 @@ int csd_apply_boundary(const csd_field* f, const int* halo, int bc, double value
 #define CSD_RED_DIFF_MAXABS 4 /* max |a-b| */
 
 /* FP64 reduction over the interior of `a` (and `b` for the DIFF ops),
- * deterministic for a given `nblocks`: pass 1 writes one partial per block
- * into the caller's device scratch `partials[nblocks]`, pass 2 writes the
- * total to the device double `*result`.  No reference counterpart: the
+ * deterministic for a given `nblocks`: pass 1 writes its blocks' sums (and the
+ * rounding errors made in them) into the caller's device scratch
+ * `partials[nblocks]`, pass 2 writes the total to the device double `*result`:
+ * the sum of the FP64 terms, rounded once in nearly all cases.  No reference counterpart: the
  * reference reduces on the host with NumPy (e.g. examples/shallow_water.py
  * energy); the B200 path keeps these global sums on the device in FP64. */
 int csd_reduce(const csd_field* a, const csd_field* b, const int* halo, int op,

@@ -43,3 +43,29 @@ def test_reduction_segments(dtype, shape, halo, nblocks):
     at = tuple(h + (s - 2 * h) // 2 for h, s in zip(halo, shape))
     ta[at] = float("nan")
     assert math.isnan(red(R.MAXABS)) and math.isnan(red(R.SUM))
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_sums_are_rounded_once(dtype):
+    """Sums of many like-signed or cancelling terms within one unit in the
+    last place of the correctly rounded sum of the FP64 terms."""
+    import torch
+
+    from cutile.runtime import reductions as R
+
+    rng = np.random.default_rng(2)
+    for shape, halo in (((300, 700), (1, 16)), ((40, 50, 60), (1, 1, 1)), ((100001,), (3,))):
+        inner = tuple(slice(h, s - h) for h, s in zip(halo, shape))
+        for offset in (1.0, 0.0):
+            a, b = ((offset + 0.1 * rng.standard_normal(shape)).astype(dtype) for _ in range(2))
+            ta, tb = torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda()
+            ia, ib = a[inner].astype(np.float64), b[inner].astype(np.float64)
+            d = ia - ib
+            for got, terms in ((R.mass(ta, halo), ia), (R.energy(ta, halo), ia * ia),
+                               (R.reduce(R.DIFF_SUMSQ, ta, halo, b=tb), d * d)):
+                want = math.fsum(terms.ravel())
+                assert abs(got.item() - want) <= np.spacing(abs(want)), (shape, offset)
+    big = torch.full((70, 70), 1e308, dtype=torch.float64, device="cuda")
+    assert R.mass(big, (1, 1)).item() == math.inf
+    big[5, 5] = -math.inf
+    assert math.isnan(R.mass(big, (1, 1)).item()) or R.mass(big, (1, 1)).item() == -math.inf
