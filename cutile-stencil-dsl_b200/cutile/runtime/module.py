@@ -207,26 +207,25 @@ class StencilProgram:
         shape = tuple(int(n) for n in shape)
         if len(shape) != self.spec["ndim"]:
             raise ValueError(f"{self.spec['name']}: expected a {self.spec['ndim']}-D shape")
-        if len(inputs) != self.spec["inputs"] or len(outputs) != self.spec["outputs"]:
-            raise TypeError(f"{self.spec['name']} takes {self.spec['inputs']} input(s) and "
-                            f"{self.spec['outputs']} output(s)")
-        for o in outputs:
-            for i in inputs:
-                if o.data_ptr() == i.data_ptr():
-                    raise ValueError("outputs must not alias inputs (the kernel reads neighbours)")
-        want = "float64" if self.spec["dtype"] in ("float64", "fp64") else "float32"
-        for t in list(inputs) + list(outputs):
-            if str(t.dtype).replace("torch.", "") != want:
-                raise TypeError(f"{self.spec['name']}: bricked field dtype {t.dtype} does not "
-                                f"match the compiled dtype {want}")
-        fin = [native.bricked_field(t, shape, bs) for t in inputs]
-        fout = [native.bricked_field(t, shape, bs) for t in outputs]
         halo = list(self.spec["halo"]) if halo is None else [int(h) for h in halo]
-        if len(halo) != len(shape):
-            raise ValueError(f"{self.spec['name']}: halo {halo} does not match the {len(shape)}-D "
-                             "shape")
-        native.launch_fields(self.kernel("bricked"), fin, fout, halo, stream,
-                             loader=loader, zchunk=zchunk, scalars=self.scalar_values(scalars))
+
+        def check():
+            if len(inputs) != self.spec["inputs"] or len(outputs) != self.spec["outputs"]:
+                raise TypeError(f"{self.spec['name']} takes {self.spec['inputs']} input(s) and "
+                                f"{self.spec['outputs']} output(s)")
+            want = "float64" if self.spec["dtype"] in ("float64", "fp64") else "float32"
+            for t in list(inputs) + list(outputs):
+                if str(t.dtype).replace("torch.", "") != want:
+                    raise TypeError(f"{self.spec['name']}: bricked field dtype {t.dtype} does not "
+                                    f"match the compiled dtype {want}")
+            if len(halo) != len(shape):
+                raise ValueError(f"{self.spec['name']}: halo {halo} does not match the "
+                                 f"{len(shape)}-D shape")
+
+        native.launch(lambda: self.kernel("bricked"), inputs, outputs, halo, stream,
+                      plans=self._plans, kind=("bricked", shape, tuple(halo)), check_fields=check,
+                      distinct=True, describe=lambda t: native.bricked_field(t, shape, bs),
+                      loader=loader, zchunk=zchunk, scalars=self.scalar_values(scalars))
 
     def launch_bricked(self, inputs, outputs, brick_size, stream=None, *,
                        scalars: dict | None = None) -> None:

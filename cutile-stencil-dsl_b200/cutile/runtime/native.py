@@ -307,18 +307,15 @@ def field_of(t, pitched: bool = False) -> Field:
         code = 1
     else:
         raise TypeError(f"unsupported dtype {t.dtype}")
-    if t.dim() < 1 or t.dim() > 3:
+    ndim, strides = t.dim(), t.stride()
+    if ndim < 1 or ndim > 3:
         raise ValueError("fields must be 1-, 2- or 3-D")
     if not t.is_contiguous():
-        if not pitched or t.stride(-1) != 1:
+        if not pitched or strides[-1] != 1:
             raise ValueError("fields must be C-contiguous")
-    f = Field()
-    f.ptr = t.data_ptr()
-    f.ndim = t.dim()
-    f.dtype = code
-    for i in range(t.dim()):
-        f.shape[i] = t.shape[i]
-        f.strides[i] = t.stride(i)
+    f = Field(t.data_ptr(), ndim, code)
+    f.shape[:ndim] = tuple(t.shape)
+    f.strides[:ndim] = strides
     return f
 
 
@@ -365,10 +362,11 @@ class LaunchPlan:
 
     __slots__ = ("kernel", "fin", "fout", "fields", "nin", "nout", "opts", "opts_ref")
 
-    def __init__(self, kernel: NativeKernel, inputs, outputs, halo, nscalars: int, kw: dict):
+    def __init__(self, kernel: NativeKernel, inputs, outputs, halo, nscalars: int, kw: dict,
+                 describe):
         self.kernel = kernel
-        self.fin = (Field * len(inputs))(*[field_of(t, True) for t in inputs])
-        self.fout = (Field * max(1, len(outputs)))(*[field_of(t, True) for t in outputs])
+        self.fin = (Field * len(inputs))(*[describe(t) for t in inputs])
+        self.fout = (Field * max(1, len(outputs)))(*[describe(t) for t in outputs])
         self.nin, self.nout = len(inputs), len(outputs)
         self.fields = ([self.fin[i] for i in range(self.nin)]
                        + [self.fout[i] for i in range(self.nout)])
@@ -392,15 +390,17 @@ def _pointer(t):
 
 
 def launch(kernel, inputs, outputs, halo, stream=None, *, plans: LaunchPlans | None = None,
-           kind=None, check_fields=None, distinct: bool = False, scalars=(), bc_value: float = 0.0,
-           dyn=None, red=None, **kw) -> None:
+           kind=None, check_fields=None, distinct: bool = False, describe=None, scalars=(),
+           bc_value: float = 0.0, dyn=None, red=None, **kw) -> None:
     """csd_launch on torch tensors.
 
     With ``plans``, what the fields' types, shapes and strides and the options
     decide -- the checks (``check_fields``) and the C structs -- is done once
     per kind of launch, ``kernel`` being a function that loads the kernel
     ``kind`` names; addresses, scalar values and the stream are read on every
-    call.  ``distinct``: outputs must not start where an input does.  Host time of
+    call.  ``distinct``: outputs must not start where an input does;
+    ``describe``: a tensor's csd_field where it is not the tensor's own shape
+    (what it depends on beside the tensor is part of ``kind``).  Host time of
     one launch call on a B200 box (two fields): 21 -> 10 us, RK4 step 104 -> 48."""
     plan = key = None
     if plans is not None:
@@ -425,7 +425,8 @@ def launch(kernel, inputs, outputs, halo, stream=None, *, plans: LaunchPlans | N
                 raise ValueError("outputs must not alias inputs (the kernel reads neighbours)")
     if plan is None:
         plan = LaunchPlan(kernel if isinstance(kernel, NativeKernel) else kernel(), inputs,
-                          outputs, halo, len(scalars), kw)
+                          outputs, halo, len(scalars), kw,
+                          describe or (lambda t: field_of(t, True)))
         if key is not None:
             if len(plans.by_kind) >= plans.LIMIT:
                 plans.by_kind.clear()
