@@ -401,7 +401,7 @@ def launch(kernel, inputs, outputs, halo, stream=None, *, plans: LaunchPlans | N
     call.  ``distinct``: outputs must not start where an input does;
     ``describe``: a tensor's csd_field where it is not the tensor's own shape
     (what it depends on beside the tensor is part of ``kind``).  Host time of
-    one launch call on a B200 box (two fields): 21 -> 10 us, RK4 step 104 -> 48."""
+    one launch call (two fields): 21 -> 10 us, RK4 step 104 -> 48."""
     plan = key = None
     if plans is not None:
         try:

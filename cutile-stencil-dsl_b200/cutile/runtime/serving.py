@@ -291,7 +291,7 @@ class StencilServer:
         """Issue one step of every active solve: one batched launch per (kind,
         dtype) group on the resident descriptors.  Groups are put together
         again only when the active solves are other ones (host time of an
-        iteration of six groups on a B200 box: 150 -> 47 us, 78 with the side
+        iteration of six groups: 150 -> 47 us, 78 with the side
         streams; 24 mixed requests of up to 60 steps, 388 launches: 12.5 ms ->
         7.8, and 6.1-7.1 with the side streams)."""
         serials = [a.serial for a in active]
@@ -318,11 +318,13 @@ class StencilServer:
             self._fork.record(stream)
             for side in lanes[1:]:
                 side.wait_event(self._fork)
-        for k, (kern, g) in enumerate(self._batch):
-            g.launch(kern, pool, handles[k % len(handles)])
-        for side, joined in zip(lanes[1:], self._joins):
-            joined.record(side)
-            stream.wait_event(joined)
+        try:
+            for k, (kern, g) in enumerate(self._batch):
+                g.launch(kern, pool, handles[k % len(handles)])
+        finally:
+            for side, joined in zip(lanes[1:], self._joins):
+                joined.record(side)
+                stream.wait_event(joined)
         self.stats.launches += len(self._batch)
 
     def _lanes(self, stream, groups: int) -> list:

@@ -55,7 +55,8 @@ typedef struct csd_launch_opts {
   int halo[3];          /* array halo width per array dim (interior = shape - 2*halo) */
   int zchunk;           /* output rows per work item along dim 0 (0 = sized at launch) */
   int grid;             /* persistent CTAs (0 = occupancy x SM count) */
-  int loader;           /* -1 auto, CSD_LOADER_TMA, CSD_LOADER_LDG */
+  int loader;           /* -1 auto (unaligned rows: the kernel's direct form where it has
+                           one, else CSD_LOADER_LDG), CSD_LOADER_TMA, CSD_LOADER_LDG */
   double bc_value;      /* Dirichlet value when the kernel fuses a boundary fill */
   uint64_t timeout_ns;  /* bound on device waits (0 = 2 s) */
   double scalars[CSD_MAX_SCALARS];  /* values of the stencil's scalar parameters */
@@ -69,7 +70,9 @@ typedef struct csd_launch_opts {
                            requests input chunk withhold_chunk - 1, so its wait runs out after
                            timeout_ns; the CTA drains its other copies and exits, and
                            csd_error_word then reports CSD_ERR_TIMEOUT.  Nothing faults or
-                           hangs: every other CTA finishes normally. */
+                           hangs: every other CTA finishes normally.  Kernels without a
+                           staging ring (register chains) wait for nothing and ignore it and
+                           timeout_ns. */
 } csd_launch_opts;
 
 /* Library version (major*100 + minor). */
