@@ -332,6 +332,20 @@ def stream_handle(stream) -> int | None:
     return getattr(stream, "cuda_stream", None) or getattr(stream, "ptr", None)
 
 
+def stream_create() -> int:
+    """A non-blocking stream of the current device (``stream_destroy`` frees
+    it once its work is done)."""
+    h = ctypes.c_void_p()
+    rc = ctypes.CDLL("libcuda.so.1").cuStreamCreate(ctypes.byref(h), 1)
+    if rc != 0:
+        raise RuntimeError(f"cuStreamCreate failed ({rc})")
+    return h.value
+
+
+def stream_destroy(handle: int) -> None:
+    ctypes.CDLL("libcuda.so.1").cuStreamDestroy_v2(ctypes.c_void_p(handle))
+
+
 def make_opts(halo, *, zchunk: int = 0, grid: int = 0, loader: int = -1, bc_value: float = 0.0,
               timeout_ns: int = 0, scalars=(), dyn=None, red=None, bc_odd=(),
               withhold_chunk: int = 0) -> LaunchOpts:

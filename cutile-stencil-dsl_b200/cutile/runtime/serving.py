@@ -28,6 +28,7 @@ from __future__ import annotations
 import itertools
 import math
 import time
+import weakref
 from collections import deque
 from dataclasses import dataclass, field
 
@@ -332,7 +333,13 @@ class StencilServer:
         import torch
 
         if groups > 1 and not self._sides:
-            self._sides = [torch.cuda.Stream(self.device) for _ in range(3)]
+            # (torch's first side stream makes a pool of them: 26 ms in the
+            # first iteration of a process, these three 0.7)
+            with torch.cuda.device(self.device):
+                handles = [native.stream_create() for _ in range(3)]
+            for h in handles:
+                weakref.finalize(self, native.stream_destroy, h)
+            self._sides = [torch.cuda.ExternalStream(h, device=self.device) for h in handles]
             self._fork = torch.cuda.Event()
             self._joins = [torch.cuda.Event() for _ in self._sides]
         return [stream, *self._sides[:groups - 1]]
