@@ -994,8 +994,10 @@ struct PlaneChainCfg {
   static constexpr int BOXW = 32 * VEC, BOXH = EY;
   static constexpr int DEPTH = 4;                    // input planes staged
   static constexpr int PLANE = EY * BOXW;            // elements of a staged plane
-  // input ring, then two planes per intermediate field
-  static constexpr int SMEM_BYTES = (DEPTH + 2 * (TEMPORAL - 1)) * NIN * PLANE * (int)sizeof(T);
+  // input ring, then two planes per intermediate field whose neighbouring rows
+  // are read
+  static constexpr int EXCHANGED = RY > 0 ? 2 * (TEMPORAL - 1) : 0;
+  static constexpr int SMEM_BYTES = (DEPTH + EXCHANGED) * NIN * PLANE * (int)sizeof(T);
   static_assert(VEC % ALIGN == 0, "a lane owns whole 16-byte vectors");
   static_assert(TX > 0 && TY > 0, "the chain consumes the whole tile");
   static_assert(RPY >= RY, "the rows on either side are the neighbouring warps'");

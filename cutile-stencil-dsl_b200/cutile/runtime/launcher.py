@@ -523,6 +523,8 @@ def register_chain_plan(radius, dtype_bytes: int, num_inputs: int, T: int, body_
     559 -> 423 (one row per thread 327 and 202 for T=2, three rows and
     eight warps 266 and 187).  Chains of several fields keep the rings (FP32
     Kahan T=2: rings 308 us, registers 345)."""
+    from cutile.passes.tiling import B200_SMEM_PER_BLOCK
+
     ndim = len(radius)
     if ndim == 3:
         rz, ry, rx = radius
@@ -531,8 +533,13 @@ def register_chain_plan(radius, dtype_bytes: int, num_inputs: int, T: int, body_
         for rows, warps, budget in ((2, 16, 84), (3, 8, 210)):
             # 32-bit registers of the T windows: own rows, rows on either side
             words = T * (rows * (2 * rz + 1) + 2 * ry * side_planes) * 4
+            # staged input planes and, for rows beside the thread's own, two
+            # planes per intermediate field (PlaneChainCfg::SMEM_BYTES)
+            planes = 4 + (2 * (T - 1) if ry > 0 else 0)
+            smem = planes * num_inputs * rows * warps * 32 * 16
             # at least half of the block's rows and columns are stored
-            if (num_inputs == 1 and words <= budget and ry <= rows and 4 * T * ry <= rows * warps
+            if (num_inputs == 1 and words <= budget and smem <= B200_SMEM_PER_BLOCK
+                    and ry <= rows and 4 * T * ry <= rows * warps
                     and 2 * (32 * vec - pad - T * rx) >= 32 * vec
                     and T * (2 * rz + 1) * rows * body_ops <= 4000):
                 return {"register_chain": vec, "chain_rows": rows, "chain_warps": warps}
