@@ -694,9 +694,8 @@ int csd_grid_item_place(const csd_grid* g, int item, int* tx, int* ty, int* z0, 
   return CSD_OK;
 }
 
-// csd_launch's own choice of copy path, and the path it may add to
-// CSD_LOADER_TMA and CSD_LOADER_LDG.
-static const int kLoaderAny = -2, kLoaderDirect = 2;
+// The path that csd_launch may add to CSD_LOADER_TMA and CSD_LOADER_LDG.
+static const int kLoaderDirect = 2;
 
 static int resident_blocks(const csd_kernel* k, int loader) {
   return loader == kLoaderDirect ? k->direct_blocks_per_sm : k->blocks_per_sm[loader];
@@ -709,8 +708,10 @@ static int item_blocks(const csd_kernel_desc& D, int items) {
   return (int)(((long long)items + per - 1) / per);
 }
 
+// `direct_ok`: an automatic choice may fall on the kernel's direct form (its
+// descriptor suits that form only).
 static int build_grid(csd_kernel* k, const csd_field* in, int n_in, const csd_field* out,
-                      int n_out, const csd_launch_opts& o, DeviceState* st, int loader_req,
+                      int n_out, const csd_launch_opts& o, DeviceState* st, bool direct_ok,
                       csd_grid* g, int* loader_out) {
   csd_kernel_desc D = k->desc;
   if (!in || (!out && n_out > 0)) return fail(CSD_EINVAL, "null field array");
@@ -785,12 +786,10 @@ static int build_grid(csd_kernel* k, const csd_field* in, int n_in, const csd_fi
   bool tma_ok = D.brick_shift == 0 ? ((g->pitch_y * esz) % 16 == 0) && ((g->pitch_z * esz) % 16 == 0)
                                    : D.brick_tma != 0;
   for (int i = 0; i < n_in; ++i) tma_ok = tma_ok && (reinterpret_cast<uintptr_t>(in[i].ptr) % 16 == 0);
-  int loader = loader_req;
-  if (loader == kLoaderAny) {   // csd_launch: the direct kernel takes unaligned rows
-    loader = tma_ok ? CSD_LOADER_TMA : k->direct ? kLoaderDirect : CSD_LOADER_LDG;
+  int loader = o.loader;
+  if (loader < 0 || loader > 1) {   // any other value: automatic
+    loader = tma_ok ? CSD_LOADER_TMA : direct_ok && k->direct ? kLoaderDirect : CSD_LOADER_LDG;
     if (loader == kLoaderDirect) D = k->direct_desc;
-  } else if (loader < 0 || loader > 1) {
-    loader = tma_ok ? CSD_LOADER_TMA : CSD_LOADER_LDG;
   }
   if (loader == CSD_LOADER_TMA && !tma_ok)
     return fail(CSD_EALIGN, "TMA path needs 16-byte aligned fields and row pitch");
@@ -904,8 +903,7 @@ int csd_launch(csd_kernel* k, const csd_field* in, int n_in, const csd_field* ou
   memset(&p, 0, sizeof(p));
   int loader = 0;
   // a withheld input chunk needs a kernel that stages chunks
-  const bool any = (o.loader < 0 || o.loader > 1) && o.withhold_chunk <= 0;
-  rc = build_grid(k, in, n_in, out, n_out, o, st, any ? kLoaderAny : o.loader, &p.g, &loader);
+  rc = build_grid(k, in, n_in, out, n_out, o, st, o.withhold_chunk <= 0, &p.g, &loader);
   if (rc) return rc;
   const csd_kernel_desc& D = loader == kLoaderDirect ? k->direct_desc : k->desc;
   p.err = reinterpret_cast<int*>(st->err);
@@ -937,7 +935,7 @@ int csd_grid_build(csd_kernel* k, const csd_field* in, int n_in, const csd_field
   rc = device_state(dev, &st);
   if (rc) return rc;
   int loader = 0;
-  rc = build_grid(k, in, n_in, out, n_out, o, st, o.loader, g, &loader);
+  rc = build_grid(k, in, n_in, out, n_out, o, st, false, g, &loader);
   if (rc) return rc;
   if (items) *items = g->items;
   if (loader_used) *loader_used = loader;
