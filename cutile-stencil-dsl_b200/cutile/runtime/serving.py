@@ -98,9 +98,10 @@ class _Group:
     Every member moves on one phase per iteration, so the descriptor list of a
     launch only takes ``P`` values while the members stay: all of them, and
     the item prefix sums, go to the device when the members change, and an
-    iteration uploads nothing."""
+    iteration uploads nothing.  A group outlives its members: it keeps their
+    number and phase, never the solves, whose fields are freed as they end."""
 
-    __slots__ = ("serials", "members", "phase0", "buf", "pinned", "items", "opts", "starts")
+    __slots__ = ("serials", "count", "phase0", "buf", "pinned", "items", "opts", "starts")
 
     def __init__(self):
         self.serials = None
@@ -111,8 +112,8 @@ class _Group:
         import numpy as np
         import torch
 
-        self.members = members
         self.serials = [a.serial for a in members]
+        self.count = len(members)
         self.phase0 = members[0].phase
         n, P = len(members), len(members[0].bufs)
         size = (P + 1) * n + 1
@@ -136,11 +137,11 @@ class _Group:
         self.opts = [native.batch_opts(native.CSD_LOADER_TMA, self.starts + 4 * ((r + 1) * n + 1))
                      for r in range(P)]
 
-    def launch(self, kern, pool_ptr: int, stream_handle) -> None:
-        P = len(self.opts)
+    def launch(self, kern, pool_ptr: int, stream_handle, phase: int) -> None:
+        """``phase``: the first member's."""
         native.check(native.library().csd_launch_batch(
-            kern.handle, pool_ptr, self.starts, len(self.members), self.items,
-            self.opts[(self.members[0].phase - self.phase0) % P], stream_handle))
+            kern.handle, pool_ptr, self.starts, self.count, self.items,
+            self.opts[(phase - self.phase0) % len(self.opts)], stream_handle))
 
 
 @dataclass
@@ -180,7 +181,8 @@ class StencilServer:
         self.device = torch.device(device)
         self._progs: dict = {}
         self._groups: dict = {}    # (kind, dtype) -> _Group
-        self._batch: list = []     # (kernel, _Group) of the current active solves
+        # (kernel, _Group, place of its first member) of the current active solves
+        self._batch: list = []
         self._serials = None       # ... which are these
         self._sides: list = []     # side streams of an iteration's launches, and their events
         self._fork = None
@@ -299,16 +301,17 @@ class StencilServer:
         if serials != self._serials:
             self._serials = serials
             members: dict = {}
-            for a in active:
-                members.setdefault((a.req.kind, a.req.dtype), []).append(a)
+            for i, a in enumerate(active):
+                members.setdefault((a.req.kind, a.req.dtype), []).append(i)
             self._batch = []
-            for key, m in members.items():
+            for key, places in members.items():
                 g = self._groups.get(key)
                 if g is None:
                     g = self._groups[key] = _Group()
+                m = [active[i] for i in places]
                 if g.serials != [a.serial for a in m]:
                     g.update(m, self.device, self.stats.iterations & 1)
-                self._batch.append((self.program(*key)[1], g))
+                self._batch.append((self.program(*key)[1], g, places[0]))
         # Groups are independent and a small one's launch is mostly latency, so
         # they go out on a few streams, all between a fork from and a join into
         # `stream`: memory is allocated, filled and reused in its order.
@@ -320,8 +323,8 @@ class StencilServer:
             for side in lanes[1:]:
                 side.wait_event(self._fork)
         try:
-            for k, (kern, g) in enumerate(self._batch):
-                g.launch(kern, pool, handles[k % len(handles)])
+            for k, (kern, g, first) in enumerate(self._batch):
+                g.launch(kern, pool, handles[k % len(handles)], active[first].phase)
         finally:
             for side, joined in zip(lanes[1:], self._joins):
                 joined.record(side)
@@ -471,6 +474,7 @@ class StencilServer:
                     else:
                         keep.append(a)
                 active = keep
+                del a            # (would hold a finished solve's fields)
                 in_flight.append((mark, finished))
             # keep one iteration in flight while the next is prepared; the
             # host time until the oldest one finishes admits arrived requests
