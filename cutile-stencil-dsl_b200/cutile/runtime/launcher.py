@@ -941,6 +941,25 @@ __all__ = ["compile", "compile_fused", "CompileResult", "pad_inner_halo",
 # --------------------------------------------------------------------------- #
 
 
+def _flux_plan(plan, fitted, dtype_bytes: int):
+    """The plan of a long 2-D flux body (``fitted``: what is left of a plan
+    after the caller's hints and the limits of shared memory).
+
+    What holds these bodies back is latency and the instruction cache (a unit
+    of four FP32 points is 30 KB of code at 16 warps per SM): 8 x 32 chunks,
+    two points per unit and the registers capped for 24 (FP64 16) warps.  20
+    shallow-water grids, 10 RK2 steps: FP32 5.10 -> 4.67 ms (two points in 8 x
+    64 chunks 5.36, one 5.75; 4 x 64 chunks 4.74), FP64 10.5 -> 9.7.  Where
+    the staged fields leave such a plan fewer than twelve warps per SM, 64-wide
+    chunks: four-field Euler fluxes in FP64 (8 warps), RK2 step, 512^2 91 us
+    against 75, 2048^2 677 against 601; in FP32 (12 warps) 46 against 53 and
+    372 against 422."""
+    wide = replace(plan, tile_x=64)
+    narrow = replace(plan, tile_x=32, threads=128, vec=2, occupancy=6 if dtype_bytes == 4 else 4)
+    p = fitted(narrow)
+    return narrow if p.threads // 32 * p.min_blocks >= 12 else wide
+
+
 def build_variants(stencil_fn, variants: dict, *, dtype: str | None = None,
                    precision: str | None = None, align_halo: bool = True,
                    tile_sizes=None, kernel_hints=None, boundary=None):
@@ -980,19 +999,16 @@ def build_variants(stencil_fn, variants: dict, *, dtype: str | None = None,
                         + (m if rk.get("w") is not None else 0))
         plan = default_engine_plan(len(stencil_halo), num_loads, dtype_bytes, stencil_halo,
                                    n_fields + extra_in, _yields(ir))
-        if len(stencil_halo) == 2 and tile_sizes is None and analysis.get("body_ops", 0) > 120:
-            # long 2-D flux bodies: what holds them back is latency and the
-            # instruction cache (a unit of four FP32 points is 30 KB of code at
-            # 16 warps per SM), so 8 x 32 chunks, two points per unit and the
-            # registers capped for 24 (FP64 16) warps.  20 shallow-water grids,
-            # 10 RK2 steps: FP32 5.10 -> 4.67 ms (two points in 8 x 64 chunks
-            # 5.36, one 5.75; 4 x 64 chunks 4.74), FP64 10.5 -> 9.7
-            plan = replace(plan, tile_x=32, threads=128, vec=2,
-                           occupancy=6 if dtype_bytes == 4 else 4)
         bmode = opts.pop("boundary_mode", "none")
-        plan = fit_plan(_plan_from(tile_sizes, kernel_hints, len(stencil_halo), plan),
-                        stencil_halo, dtype_bytes, n_fields + extra_in,
-                        analysis.get("body_ops", 0), periodic=bmode == "periodic")
+
+        def fitted(p):
+            return fit_plan(_plan_from(tile_sizes, kernel_hints, len(stencil_halo), p),
+                            stencil_halo, dtype_bytes, n_fields + extra_in,
+                            analysis.get("body_ops", 0), periodic=bmode == "periodic")
+
+        if len(stencil_halo) == 2 and tile_sizes is None and analysis.get("body_ops", 0) > 120:
+            plan = _flux_plan(plan, fitted, dtype_bytes)
+        plan = fitted(plan)
         verify_engine_plan(clone, plan, stencil_halo, dtype_bytes, n_fields + extra_in,
                            periodic=bmode == "periodic")
         target = lower_to_target_ir(ir.clone(), plan.tile_sizes(), tuple(halo_widths),
