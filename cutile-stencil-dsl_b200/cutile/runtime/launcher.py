@@ -941,7 +941,7 @@ __all__ = ["compile", "compile_fused", "CompileResult", "pad_inner_halo",
 # --------------------------------------------------------------------------- #
 
 
-def _flux_plan(plan, fitted, dtype_bytes: int):
+def _flux_plan(plan, fitted, dtype_bytes: int, hinted: bool):
     """The plan of a long 2-D flux body (``fitted``: what is left of a plan
     after the caller's hints and the limits of shared memory).
 
@@ -953,8 +953,10 @@ def _flux_plan(plan, fitted, dtype_bytes: int):
     the staged fields leave such a plan fewer than twelve warps per SM, 64-wide
     chunks: four-field Euler fluxes in FP64 (8 warps), RK2 step, 512^2 91 us
     against 75, 2048^2 677 against 601; in FP32 (12 warps) 46 against 53 and
-    372 against 422."""
+    372 against 422.  Callers' hints refine the 64-wide plan."""
     wide = replace(plan, tile_x=64)
+    if hinted:
+        return wide
     narrow = replace(plan, tile_x=32, threads=128, vec=2, occupancy=6 if dtype_bytes == 4 else 4)
     p = fitted(narrow)
     return narrow if p.threads // 32 * p.min_blocks >= 12 else wide
@@ -1007,7 +1009,7 @@ def build_variants(stencil_fn, variants: dict, *, dtype: str | None = None,
                             analysis.get("body_ops", 0), periodic=bmode == "periodic")
 
         if len(stencil_halo) == 2 and tile_sizes is None and analysis.get("body_ops", 0) > 120:
-            plan = _flux_plan(plan, fitted, dtype_bytes)
+            plan = _flux_plan(plan, fitted, dtype_bytes, bool(kernel_hints))
         plan = fitted(plan)
         verify_engine_plan(clone, plan, stencil_halo, dtype_bytes, n_fields + extra_in,
                            periodic=bmode == "periodic")

@@ -38,3 +38,14 @@ def test_narrow_chunks_keep_twelve_warps(fn, dtype, tile_x):
         assert p.vec == (2 if tile_x == 32 else 16 // (4 if dtype == "float32" else 8))
         if tile_x == 32:
             assert p.threads // 32 * p.min_blocks >= 12
+
+
+@pytest.mark.parametrize("dtype", ["float32", "float64"])
+def test_hints_refine_the_64_wide_plan(dtype):
+    """A caller's threads, stages or occupancy mean what they mean for every
+    other body: the narrow plan's blocks hold 128 threads at most."""
+    vec = 16 // (4 if dtype == "float32" else 8)
+    for p in _plans(D.sw_rhs, dtype, kernel_hints={"threads": 64}):
+        assert (p.tile_x, p.vec, p.threads, p.occupancy) == (64, vec, 64, 0)
+    for p in _plans(D.sw_rhs, dtype, kernel_hints={"min_blocks": 2}):
+        assert (p.tile_x, p.vec, p.occupancy) == (64, vec, 2)
