@@ -79,8 +79,9 @@ def _parse_line(line: str):
 
 
 class _BodyEmitter:
-    def __init__(self, prefix: str):
+    def __init__(self, prefix: str, shared_divisors=frozenset()):
         self.prefix = prefix
+        self.shared_divisors = shared_divisors   # scalars whose reciprocal is kept
         self.types: dict[str, str] = {}
         self.consts: dict[str, float] = {}
         self.lines: list[str] = []
@@ -88,21 +89,20 @@ class _BodyEmitter:
 
     def divide(self, x: str, y: str, tgt: str) -> str:
         """``x / y``, correctly rounded: by a power of two as the product with
-        its exact reciprocal, in FP64 by another constant or a scalar parameter
-        through a divisor that its quotients share, else a full division (in
+        its exact reciprocal, in FP64 by a scalar of ``shared_divisors``
+        through the divisor that its quotients share, else a full division (in
         FP32 that is as short: shallow-water RK2 batch 5.10 ms, 5.58 with shared
-        divisors; FP64 12.3 -> 10.4)."""
+        divisors).  A constant takes the full division too, full -> by its
+        reciprocal: 4096^2 FP64, a quotient by 12 per point, 66 -> 72 us, an RK4
+        step of it on 2048^2 117 -> 136, 256^3 by 6 55 -> 62."""
         ct = _CTYPE[tgt]
         if self.types.get(y) == "w" and y in self.consts:
             v = self.consts[y]
-            if math.isfinite(v) and 2.0 ** -60 <= abs(v) < 2.0 ** 60:
-                if abs(math.frexp(v)[0]) == 0.5:
-                    fn = "__fmul_rn" if tgt == "f32" else "__dmul_rn"
-                    return f"{fn}({x}, {hex_literal(1.0 / v, ct)})"
-                if tgt == "f64":
-                    return (f"csd::div_by({x}, csd::Divisor{{{hex_literal(v)}, "
-                            f"{hex_literal(1.0 / v)}, true}})")
-        if tgt == "f64" and y[0] == "s" and y[1:].isdigit():
+            if (math.isfinite(v) and 2.0 ** -60 <= abs(v) < 2.0 ** 60
+                    and abs(math.frexp(v)[0]) == 0.5):
+                fn = "__fmul_rn" if tgt == "f32" else "__dmul_rn"
+                return f"{fn}({x}, {hex_literal(1.0 / v, ct)})"
+        if tgt == "f64" and y in self.shared_divisors:
             decl = f"const csd::Divisor div_{y} = csd::divisor({self.conv(y, tgt)});"
             if decl not in self.divisors:
                 self.divisors.append(decl)
@@ -213,6 +213,27 @@ class _ShiftClasses:
         if cid is None:
             cid = self.ids[key] = len(self.ids)
         return cid
+
+
+def _shared_divisors(ssa: list, accesses: list, points: int) -> frozenset:
+    """Scalar parameters that an FP64 body of ``points`` points divides by
+    often enough for a kept reciprocal to pay: twice per point.  Footprints of
+    more than 16 loads are at the register limit already and keep full
+    divisions.  B200, full -> shared: four quotients by dx per point (diffusion,
+    4096^2) 114 -> 99 us, two 68 -> 63, one 68 -> 68; shallow water with six,
+    RK2 batch, 12.3 -> 10.5 ms; four-field Euler fluxes (20 loads), RK2 step on
+    2048^2, 601 -> 633 us."""
+    per_field: dict = {}
+    for f, *offs in accesses:
+        per_field.setdefault(f, []).append(any(offs))
+    if sum(len(v) for v in per_field.values() if any(v)) > 16:
+        return frozenset()
+    count: dict = {}
+    for raw in ssa:
+        _, op, args, _, _ = _parse_line(raw)
+        if op == "divf" and args[1][0] == "s" and args[1][1:].isdigit():
+            count[args[1]] = count.get(args[1], 0) + 1
+    return frozenset(s for s, n in count.items() if n >= 2 * points)
 
 
 def emit_body(kernel: KernelOp, vec: int | None = None, suffix: str = "",
@@ -335,7 +356,7 @@ def emit_body(kernel: KernelOp, vec: int | None = None, suffix: str = "",
                                    f"{tail} : {typ}")
                 for res, idx in rets:
                     stores.append((m if idx is None else idx, j * vec + k, rename(res, info, j, k)))
-    em = _BodyEmitter("q_")
+    em = _BodyEmitter("q_", _shared_divisors(ssa, accesses, vec * rpy) if field_t == "f64" else ())
     em.emit(ssa, access_types)
     for line in em.divisors + em.lines:
         out.append("    " + line)
