@@ -8,6 +8,7 @@ is missing the calls raise.
 
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import os
 import threading
@@ -332,6 +333,22 @@ def stream_handle(stream) -> int | None:
     return getattr(stream, "cuda_stream", None) or getattr(stream, "ptr", None)
 
 
+def on_stream(stream):
+    """A context in which torch allocates and launches on ``stream`` (what the
+    entry points take; None: the current one): scratch that is filled and
+    reused in the order of the kernels that use it."""
+    if stream is None:
+        return contextlib.nullcontext()
+    import torch
+
+    if isinstance(stream, torch.cuda.Stream):
+        return torch.cuda.stream(stream)
+    handle = stream_handle(stream)
+    if handle in (None, 0, 1):     # the default stream, also by its legacy name
+        return torch.cuda.stream(torch.cuda.default_stream())
+    return torch.cuda.stream(torch.cuda.ExternalStream(handle))
+
+
 def stream_create() -> int:
     """A non-blocking stream of the current device (``stream_destroy`` frees
     it once its work is done)."""
@@ -653,6 +670,6 @@ def error_word(reset: bool = True) -> int:
 
 __all__ = ["library", "check", "compile_source", "NativeModule", "NativeKernel", "launch",
            "apply_boundary", "error_word", "error_status", "CSD_ETIMEOUT", "CSD_ERR_TIMEOUT", "CsdError", "field_of", "default_cache_dir",
-           "make_opts", "LaunchPlans", "grid_build_rotations", "batch_opts", "grid_size", "grid_build", "launch_batch", "bricked_shape",
+           "make_opts", "LaunchPlans", "on_stream", "grid_build_rotations", "batch_opts", "grid_size", "grid_build", "launch_batch", "bricked_shape",
            "to_bricks", "from_bricks", "bricked_field", "launch_fields",
            "GridHead", "plan_items", "NVCC_OPTIONS", "find_nvcc", "aot_compile", "read_image", "CSD_LOADER_TMA", "CSD_LOADER_LDG", "BC_MODES"]

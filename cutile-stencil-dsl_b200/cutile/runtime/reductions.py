@@ -10,42 +10,29 @@ the device as 0-d float64 tensors (read them with ``.item()`` when needed).
 from __future__ import annotations
 
 import ctypes
-import threading
 
 from cutile.runtime import native
 
 SUM, SUMSQ, MAXABS, DIFF_SUMSQ, DIFF_MAXABS = 0, 1, 2, 3, 4
 DEFAULT_BLOCKS = 296  # 2 per SM on B200; fixed so results do not depend on the device
 
-_scratch: dict = {}
-_lock = threading.Lock()
-
-
-def _partials(device, nblocks: int):
-    import torch
-
-    key = (device, nblocks)
-    with _lock:
-        buf = _scratch.get(key)
-        if buf is None:
-            buf = torch.empty(nblocks, dtype=torch.float64, device=device)
-            _scratch[key] = buf
-    return buf
-
-
 def reduce(op: int, a, halo, b=None, out=None, stream=None, nblocks: int = DEFAULT_BLOCKS,
            partials=None):
-    """Generic entry: ``op`` over the interior of ``a`` (and ``b``)."""
+    """Generic entry: ``op`` over the interior of ``a`` (and ``b``).
+
+    The partials are the call's own (unless given) and are reused in
+    ``stream``'s order: reductions on several streams or threads overlap."""
     import torch
 
     lib = native.library()
     fa = native.field_of(a)
     fb = native.field_of(b) if b is not None else None
     h = (ctypes.c_int * 3)(*([int(x) for x in halo] + [0] * (3 - len(halo))))
-    if out is None:
-        out = torch.empty((), dtype=torch.float64, device=a.device)
-    if partials is None:
-        partials = _partials(a.device, nblocks)
+    with native.on_stream(stream):
+        if out is None:
+            out = torch.empty((), dtype=torch.float64, device=a.device)
+        if partials is None:
+            partials = torch.empty(nblocks, dtype=torch.float64, device=a.device)
     native.check(lib.csd_reduce(ctypes.byref(fa), ctypes.byref(fb) if fb is not None else None,
                                 h, op, ctypes.c_void_p(partials.data_ptr()), nblocks,
                                 ctypes.c_void_p(out.data_ptr()),
@@ -67,7 +54,9 @@ def residual(a, b, halo, **kw):
     """L2 norm of ``a - b`` over the interior (FP64, sqrt taken on the device)."""
     import torch
 
-    return torch.sqrt(reduce(DIFF_SUMSQ, a, halo, b=b, **kw))
+    total = reduce(DIFF_SUMSQ, a, halo, b=b, **kw)
+    with native.on_stream(kw.get("stream")):
+        return torch.sqrt(total)
 
 
 def max_abs(u, halo, **kw):
