@@ -153,7 +153,7 @@ def _module_code(name: str, method: str, cuda: str, info: dict) -> str:
     e.line(f"def rk_{method}_solve(u0, dt, num_steps, stream=None, **scalars):")
     with e.indent():
         e.line(f'"""Run {method.upper()} for ``num_steps`` steps from a copy of ``u0``."""')
-        e.line("u = _PROGRAM.copy_state(u0)")
+        e.line("u = _PROGRAM.copy_state(u0, stream)")
         e.line("for _ in range(num_steps):")
         with e.indent():
             e.line("_PROGRAM.step(u, dt, stream, scalars)")

@@ -31,7 +31,6 @@ class RKProgram:
         self._lock = threading.Lock()
         self._plans = native.LaunchPlans()
         self._work: dict = {}
-        self._dt: dict = {}
         self.bc_odd: tuple = ()
         self.bc_value = 0.0
 
@@ -48,8 +47,9 @@ class RKProgram:
         return m.kernel(self.spec["stages"][stage])
 
     # -- buffers -------------------------------------------------------------
-    def copy_state(self, u0):
-        t = tuple(x.clone() for x in _as_tuple(u0))
+    def copy_state(self, u0, stream=None):
+        with native.on_stream(stream):
+            t = tuple(x.clone() for x in _as_tuple(u0))
         return t if isinstance(u0, (tuple, list)) else t[0]
 
     def workspace(self, state: tuple) -> dict:
@@ -91,27 +91,26 @@ class RKProgram:
     def step(self, u, dt, stream=None, scalars: dict | None = None, aux=()) -> None:
         """One RK step of the state ``u`` in place; ``dt`` is a float or a
         device float64 tensor of one element."""
-        import torch
-
         fields = _as_tuple(u)
         m = self.spec["state_fields"]
         if len(fields) + len(aux) != self.spec["fields"]:
             raise TypeError(f"the operator reads {self.spec['fields']} fields")
-        state = fields[:m]
-        if isinstance(dt, torch.Tensor):
-            dyn = dt
-        else:
-            dyn = self._dt.get(state[0].device)
-            if dyn is None:
-                dyn = torch.empty(1, dtype=torch.float64, device=state[0].device)
-                self._dt[state[0].device] = dyn
-            dyn.fill_(float(dt))
+        # dt, the workspace's first zeros and the final copy are part of the
+        # step: in its stream's order, with a dt scalar of the step's own
+        with native.on_stream(stream):
+            self._step(fields[:m], tuple(fields[m:]) + tuple(aux), dt, stream, scalars)
+
+    def _step(self, state: tuple, rest: tuple, dt, stream, scalars: dict | None) -> None:
+        import torch
+
+        dyn = dt if isinstance(dt, torch.Tensor) else torch.full(
+            (1,), float(dt), dtype=torch.float64, device=state[0].device)
         bufs = dict(self.workspace(state))
         bufs["u"] = state
         sv = self._scalars(scalars)
         halo = self.spec["halo"]
         for k in range(len(self.table)):
-            inputs, outputs = self.stage_io(k, bufs, tuple(fields[m:]) + tuple(aux))
+            inputs, outputs = self.stage_io(k, bufs, rest)
             native.launch(lambda: self.kernel(k), inputs, outputs, halo, stream,  # noqa: B023
                           plans=self._plans, kind=k, scalars=sv, dyn=dyn,
                           bc_odd=tuple(self.bc_odd), bc_value=self.bc_value)
