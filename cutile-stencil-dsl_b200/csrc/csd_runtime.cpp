@@ -349,6 +349,10 @@ struct csd_kernel {
   CUfunction direct = nullptr;
   csd_kernel_desc direct_desc;
   int direct_blocks_per_sm = 0;
+  // a register chain's ring form, the faster one on arrays of fewer than
+  // ring_below rows of the chain's tiles (csd_launch), when its module has one
+  csd_kernel* ring = nullptr;
+  long long ring_below = 0;
   std::string name;
 };
 
@@ -491,7 +495,25 @@ int csd_kernel_get(csd_module* m, const char* name, csd_kernel** out) {
                                                     k->direct_desc.threads, 0) == 0 &&
       k->direct_blocks_per_sm > 0)
     k->direct = direct;
+  long long below = 0;
+  if (d.cuModuleGetGlobal(&dp, &sz, m->mod, (n + "_ring_below").c_str()) == 0 &&
+      sz == sizeof(below) && d.cuMemcpyDtoH(&below, dp, sizeof(below)) == 0 && below > 0) {
+    const int rc = csd_kernel_get(m, (n + "_ring").c_str(), &k->ring);
+    if (rc) {
+      delete k;
+      return rc;
+    }
+    k->ring->name = n;
+    k->ring_below = below;
+  }
   *out = k;
+  return CSD_OK;
+}
+
+int csd_kernel_ring(const csd_kernel* k, csd_kernel** ring, long long* below) {
+  if (!k || !ring || !below) return fail(CSD_EINVAL, "null argument");
+  *ring = k->ring;
+  *below = k->ring_below;
   return CSD_OK;
 }
 
@@ -905,6 +927,18 @@ int csd_launch(csd_kernel* k, const csd_field* in, int n_in, const csd_field* ou
   // a withheld input chunk needs a kernel that stages chunks
   rc = build_grid(k, in, n_in, out, n_out, o, st, o.withhold_chunk <= 0, &p.g, &loader);
   if (rc) return rc;
+  // a chain's items and copies may be asked for by zchunk and loader; left to
+  // the library, arrays that are small for it take the rings.  Rows that are
+  // not aligned cost the rings' per-element copies more (radius-2 FP32 T=5,
+  // rings / registers us: 257 x 259 25 / 27, 513 x 515 49 / 33, aligned 512^2
+  // 25 / 33), so a quarter of the size decides there.
+  const long long limit = loader == CSD_LOADER_TMA ? k->ring_below : k->ring_below / 4;
+  if (k->ring && (o.loader < 0 || o.loader > 1) && o.zchunk <= 0 && o.withhold_chunk <= 0 &&
+      (long long)p.g.tiles[0] * p.g.tiles[1] * p.g.interior[0] < limit) {
+    k = k->ring;
+    rc = build_grid(k, in, n_in, out, n_out, o, st, false, &p.g, &loader);
+    if (rc) return rc;
+  }
   const csd_kernel_desc& D = loader == kLoaderDirect ? k->direct_desc : k->desc;
   p.err = reinterpret_cast<int*>(st->err);
   p.timeout_ns = o.timeout_ns ? o.timeout_ns : 2000000000ull;

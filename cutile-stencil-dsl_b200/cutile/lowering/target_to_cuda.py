@@ -484,8 +484,9 @@ def _internal_radius(ndim: int, radius) -> tuple[int, int, int]:
     return (0, 0, r[0])
 
 
-def engine_params(kernel: KernelOp) -> dict:
-    """Template parameters of the engine instance described by *kernel*."""
+def engine_params(kernel: KernelOp, ring: bool = False) -> dict:
+    """Template parameters of the engine instance described by *kernel*
+    (``ring``: of a register chain's ring form)."""
     ndim = kernel.ndim.data
     dtype = kernel.dtype.data
     tile = [a.data for a in kernel.tile_shape.data]
@@ -493,6 +494,9 @@ def engine_params(kernel: KernelOp) -> dict:
     if kernel.kernel_hints is not None:
         items = [a.data for a in kernel.kernel_hints.data]
         hints = {k: eval(v, {}) for k, v in zip(items[0::2], items[1::2])}  # repr'd ints
+    if ring:
+        hints.pop("register_chain", None)
+        hints.pop("chain_rows", None)
     if ndim == 3:
         rows, ty, tx = tile
     elif ndim == 2:
@@ -524,6 +528,8 @@ def engine_params(kernel: KernelOp) -> dict:
         "OCCUPANCY": int(hints.get("occupancy", 0)),   # a caller's blocks per SM (0: none)
         # points per lane of a register chain (0: the ring engine)
         "CHAIN": int(hints.get("register_chain", 0)),
+        # rows of its tiles from which the chain is the faster form (0: always)
+        "RING_BELOW": int(hints.get("ring_below", 0)),
         "VEC": int(hints.get("register_chain", 0)
                    or hints.get("vec", 4 if dtype in ("float32", "fp32") else 2)),
     }
@@ -558,6 +564,41 @@ def _brick_code(kernel: KernelOp, ndim: int) -> int:
     return (ndim << 4) | (b.bit_length() - 1)
 
 
+def _emit_engine(name: str, p: dict) -> list:
+    """The ``<name>_tma`` and ``<name>_ldg`` kernels and their descriptor."""
+    parts = []
+    brick_tma = brick_tma_eligible(p)
+    for suffix, loader in (("tma", "CSD_LOADER_TMA"), ("ldg", "CSD_LOADER_LDG")):
+        if p["BRICK"] and not brick_tma:
+            loader = "CSD_LOADER_LDG"   # bricked fields the TMA boxes cannot stage
+        entry, nt, minb = "stream_engine", p["NT"], p["MINB"]
+        cfg = (f"csd::Cfg<{p['T']}, {p['NIN']}, {p['NOUT']}, {p['RZ']}, {p['RY']}, {p['RX']}, "
+               f"{p['ROWS']}, {p['TY']}, {p['TX']}, {p['NT']}, {p['STAGES']}, {p['TEMPORAL']}, "
+               f"{loader}, {p['BC']}, {p['REDUCE']}, {p['BRICK']}, {p['RPY']}, {p['VEC']}>")
+        if p["CHAIN"]:
+            entry, nt, minb = "register_chain", 32 * p["CHAIN_WARPS"], 1
+            cfg = (f"csd::ChainCfg<{p['T']}, {p['NIN']}, {p['NOUT']}, {p['RZ']}, {p['RX']}, "
+                   f"{nt}, {p['TEMPORAL']}, {loader}, {p['VEC']}>")
+            if p["ndim"] == 3:
+                entry = "plane_chain"
+                cfg = (f"csd::PlaneChainCfg<{p['T']}, {p['NIN']}, {p['NOUT']}, {p['RZ']}, "
+                       f"{p['RY']}, {p['RX']}, {nt}, {p['TEMPORAL']}, {loader}, {p['VEC']}, "
+                       f"{p['RPY']}>")
+        parts.append(f"typedef {cfg} Cfg_{name}_{suffix};")
+        parts.append(f'extern "C" __global__ void __launch_bounds__({nt}, {minb})')
+        parts.append(f"{name}_{suffix}(const __grid_constant__ csd_params p) {{")
+        parts.append(f"  csd::{entry}<Cfg_{name}_{suffix}, Body_{name}>(p);")
+        parts.append("}")
+    c = f"Cfg_{name}_tma"
+    # both entries launch with one shared-memory size: the larger one
+    smem = (f"({c}::SMEM_BYTES > Cfg_{name}_ldg::SMEM_BYTES ? {c}::SMEM_BYTES : "
+            f"Cfg_{name}_ldg::SMEM_BYTES)")
+    parts.append(_descriptor(f"{name}_desc", c, p, p["ZCHUNK"], p["MINB"],
+                             1 if brick_tma else 0, smem))
+    parts.append("")
+    return parts
+
+
 def emit_cuda(module: ModuleOp, preamble: bool = True) -> str:
     """CUDA translation unit for the kernel(s) in a D3 module (``preamble=False``
     gives just the kernels, to append to another unit)."""
@@ -582,35 +623,16 @@ def emit_cuda(module: ModuleOp, preamble: bool = True) -> str:
         parts.append(f"// expression: {kernel.expression.data}")
         parts.append(emit_body(kernel))
         parts.append("")
-        brick_tma = brick_tma_eligible(p)
-        for suffix, loader in (("tma", "CSD_LOADER_TMA"), ("ldg", "CSD_LOADER_LDG")):
-            if p["BRICK"] and not brick_tma:
-                loader = "CSD_LOADER_LDG"   # bricked fields the TMA boxes cannot stage
-            entry, nt, minb = "stream_engine", p["NT"], p["MINB"]
-            cfg = (f"csd::Cfg<{p['T']}, {p['NIN']}, {p['NOUT']}, {p['RZ']}, {p['RY']}, {p['RX']}, "
-                   f"{p['ROWS']}, {p['TY']}, {p['TX']}, {p['NT']}, {p['STAGES']}, {p['TEMPORAL']}, "
-                   f"{loader}, {p['BC']}, {p['REDUCE']}, {p['BRICK']}, {p['RPY']}, {p['VEC']}>")
-            if p["CHAIN"]:
-                entry, nt, minb = "register_chain", 32 * p["CHAIN_WARPS"], 1
-                cfg = (f"csd::ChainCfg<{p['T']}, {p['NIN']}, {p['NOUT']}, {p['RZ']}, {p['RX']}, "
-                       f"{nt}, {p['TEMPORAL']}, {loader}, {p['VEC']}>")
-                if p["ndim"] == 3:
-                    entry = "plane_chain"
-                    cfg = (f"csd::PlaneChainCfg<{p['T']}, {p['NIN']}, {p['NOUT']}, {p['RZ']}, "
-                           f"{p['RY']}, {p['RX']}, {nt}, {p['TEMPORAL']}, {loader}, {p['VEC']}, "
-                           f"{p['RPY']}>")
-            parts.append(f"typedef {cfg} Cfg_{name}_{suffix};")
-            parts.append(f'extern "C" __global__ void __launch_bounds__({nt}, {minb})')
-            parts.append(f"{name}_{suffix}(const __grid_constant__ csd_params p) {{")
-            parts.append(f"  csd::{entry}<Cfg_{name}_{suffix}, Body_{name}>(p);")
-            parts.append("}")
-        c = f"Cfg_{name}_tma"
-        # both entries launch with one shared-memory size: the larger one
-        smem = (f"({c}::SMEM_BYTES > Cfg_{name}_ldg::SMEM_BYTES ? {c}::SMEM_BYTES : "
-                f"Cfg_{name}_ldg::SMEM_BYTES)")
-        parts.append(_descriptor(f"{name}_desc", c, p, p["ZCHUNK"], p["MINB"],
-                                 1 if brick_tma else 0, smem))
-        parts.append("")
+        parts.extend(_emit_engine(name, p))
+        if p["CHAIN"] and p["RING_BELOW"] > 0:
+            # the same steps by the shared-memory rings, for smaller arrays
+            q = engine_params(kernel, ring=True)
+            parts.append(emit_body(kernel, q["VEC"], "_ring"))
+            parts.append("")
+            parts.extend(_emit_engine(f"{name}_ring", q))
+            parts.append(f'extern "C" __device__ const long long {name}_ring_below = '
+                         f'{p["RING_BELOW"]};')
+            parts.append("")
         if direct_plan(kernel)[0]:
             parts.extend(_emit_direct(kernel))
     return "\n".join(parts) + "\n"

@@ -502,27 +502,69 @@ def _side_planes(ir) -> int:
     return max((lead - o[0] + 1 for o in offs if o[1] != 0), default=0)
 
 
+def _quotients(ir) -> bool:
+    """Whether the body divides field values by anything but a power of two
+    (which is a product)."""
+    from cutile.dialects import arith as A
+    from cutile.dialects.stencil import AccessOp
+
+    fields, constants = set(), {}
+    for op in ir.walk():
+        out = [id(r) for r in op.results]
+        if isinstance(op, AccessOp) or any(id(x) in fields for x in op.operands):
+            fields.update(out)
+        if isinstance(op, A.ConstantOp):
+            constants[out[0]] = float(op.properties["value"].value.data)
+        if isinstance(op, A.DivfOp) and out[0] in fields:
+            y = constants.get(id(op.operands[1]))
+            if y is None or not math.isfinite(y) or abs(math.frexp(y)[0]) != 0.5:
+                return True
+    return False
+
+
 def register_chain_plan(radius, dtype_bytes: int, num_inputs: int, T: int, body_ops: int,
-                        side_planes: int = 0) -> dict:
+                        side_planes: int = 0, num_loads: int = 0, quotients: bool = False) -> dict:
     """Hints of the register chain (engine.cuh ``ChainCfg``,
-    ``PlaneChainCfg``) for a chain of T steps: points per lane, and in 3-D rows
-    per thread and warps per block; {} where the shared-memory rings keep it.
+    ``PlaneChainCfg``) for a chain of T steps: points per lane, in 3-D rows
+    per thread and warps per block, and ``ring_below``, the size under which a
+    launch takes the shared-memory rings after all (0: never); {} where the
+    rings are the only form.
 
-    1-D and 2-D chains whose windows fit the registers take it.  Measured on
-    B200 per launch, rings -> registers: heat 1024^2 FP64 T=5 103 -> 10.9 us,
-    4096^2 323 -> 68; FP32 T=8 194 -> 13.2 and 472 -> 62; Kahan T=4 80 -> 12.6
-    and 275 -> 73; radius 2 FP64 T=4 80 -> 25 and 315 -> 170; heat1d 2^22 T=8
-    FP64 123 -> 18, FP32 68 -> 10.  The one loss seen is a radius-2 FP32 chain
-    of three or four steps on a grid too small to fill the chip (200 x 300:
-    8.5 -> 9.9 and 12.2 -> 16.0 us; 1024^2: 28 -> 15 and 51 -> 28).
+    Chains whose windows fit the registers take them.  Measured on B200 per
+    launch, rings -> registers: heat 1024^2 FP64 T=5 103 -> 10.9 us, 4096^2 323
+    -> 68; FP32 T=8 194 -> 13.2 and 472 -> 62; Kahan T=4 80 -> 12.6 and 275 ->
+    73; heat1d 2^22 T=8 FP64 123 -> 18, FP32 68 -> 10; 7-point 384^3 FP64 T=2
+    329 -> 212, T=4 982 -> 487; FP32 T=2 186 -> 148, T=4 559 -> 423.
 
-    3-D chains take it as far as their windows fit: two rows per thread and
-    sixteen warps while a block of them keeps 128 registers each, else three
-    rows and eight warps.  7-point 384^3 per launch, rings -> registers: FP64
-    T=2 329 -> 212 us, T=4 982 -> 487; FP32 T=2 186 -> 148, T=4
-    559 -> 423 (one row per thread 327 and 202 for T=2, three rows and
-    eight warps 266 and 187).  Chains of several fields keep the rings (FP32
-    Kahan T=2: rings 308 us, registers 345)."""
+    An item computes T rz rows more than it stores on either side, so a chain
+    has to have enough rows of its tiles (tiles across X and Y, times the rows
+    or planes of each: ``ring_below`` counts these) for long items; the rings
+    share such rows between the threads of a block.  Ratio rings / registers:
+    * radius 1 without quotients (5 and 9 points, 1-D, T = 2 to 8): 1.0 and
+      more from 64^2 on, so always registers;
+    * 9-point stars of radius 2: FP64 T <= 4 1.0 and more everywhere, T = 6 0.92
+      at 256^2 (1280 tile rows) and 1.2 at 384^2 (2688); FP32 T = 2 1.05 and
+      more, T = 3 to 6 0.7 to 0.9 from 256^2 to 512^2 (2560), 1.1 to 1.6 at
+      768^2 (5376), 1.8 to 2.5 at 4096 x 20 (4096);
+    * denser footprints, radius 3, FP32 quotients at radius 2: FP64 0.3 to 1.1
+      up to 512^2 (5120), 1.04 to 1.8 at 768^2 (10752); FP32 T = 2 0.7 to 1.05
+      up to 4000 x 300 (12000), 1.0 to 2.3 at 1448^2 and 16384 x 64 (16384), T >=
+      3 0.4 to 0.9 up to 768^2, 1.02 to 1.5 at 1024^2 (9216);
+    * quotients at radius 1: FP32 0.85 at 512^2, 1.0 to 1.7 at 768^2; FP64 T >= 4
+      0.6 to 1.1 up to 512^2 (4608), 1.2 to 1.6 at 768^2 (10752), T <= 3 0.9 at
+      4096^2; at radius 2 FP64 0.7 to 0.9 at 4096^2: a full division's branches
+      stop the overlap of the stages that the registers live on;
+    * 3-D: FP64 0.8 to 1.0 at 48^3 (96 tile planes), 1.0 to 1.5 at 64^3 (384);
+      FP32 0.65 to 1.0 at 64^3 (192 to 256), 1.0 to 3.0 at 96^3 (384); pointwise and
+      X-only bodies with T = 2 0.5 to 0.9 at 512 x 8 x 512 (4608), 1.0 to 1.3 at
+      256^3 (10240); with quotients 0.3 to 0.5 at 256^3 in FP64, 0.9 to 1.0 in
+      FP32.
+
+    In 3-D two rows per thread and sixteen warps while a block of them keeps
+    128 registers each, else three rows and eight warps (one row per thread
+    327 and 202 us for T=2 above, three rows and eight warps 266 and 187).
+    3-D chains of several fields keep the rings (FP32 Kahan T=2: rings 308 us,
+    registers 345)."""
     from cutile.passes.tiling import B200_SMEM_PER_BLOCK
 
     ndim = len(radius)
@@ -530,6 +572,7 @@ def register_chain_plan(radius, dtype_bytes: int, num_inputs: int, T: int, body_
         rz, ry, rx = radius
         vec = 16 // dtype_bytes
         pad = -(-T * rx // vec) * vec
+        below = 8192 if rz == 0 and ry == 0 and T == 2 else 288
         for rows, warps, budget in ((2, 16, 84), (3, 8, 210)):
             # 32-bit registers of the T windows: own rows, rows on either side
             words = T * (rows * (2 * rz + 1) + 2 * ry * side_planes) * 4
@@ -538,25 +581,41 @@ def register_chain_plan(radius, dtype_bytes: int, num_inputs: int, T: int, body_
             planes = 4 + (2 * (T - 1) if ry > 0 else 0)
             smem = planes * num_inputs * rows * warps * 32 * 16
             # at least half of the block's rows and columns are stored
-            if (num_inputs == 1 and words <= budget and smem <= B200_SMEM_PER_BLOCK
+            if (num_inputs == 1 and not quotients and words <= budget
+                    and smem <= B200_SMEM_PER_BLOCK
                     and ry <= rows and 4 * T * ry <= rows * warps
                     and 2 * (32 * vec - pad - T * rx) >= 32 * vec
                     and T * (2 * rz + 1) * rows * body_ops <= 4000):
-                return {"register_chain": vec, "chain_rows": rows, "chain_warps": warps}
+                return {"register_chain": vec, "chain_rows": rows, "chain_warps": warps,
+                        "ring_below": below}
         return {}
     rz, rx = (radius[0] if ndim == 2 else 0), radius[-1]
+    r, fp64 = max(rz, rx), dtype_bytes == 8
     # one 16-byte vector per lane; two in 1-D, where no rows are kept (FP32
     # 2^22: 14.8 us with one, 10.1 with two, 10.2 with four)
     vec = 16 // dtype_bytes * (2 if ndim == 1 else 1)
     # registers of the T windows (192: two blocks per SM still beat the rings,
     # Kahan T=8 1094 -> 139 us at 4096^2; past that they spill), and the
-    # unrolled code (2 rz + 1 copies of every stage's body)
+    # unrolled code (2 rz + 1 copies of every stage's body; 25 points of radius
+    # 2 at 4096^2, FP64: 1860 ops 954 -> 787 us, 2170 ops 1175 -> 1451)
     window = T * num_inputs * (2 * rz + 1) * vec * dtype_bytes // 4
-    if window > 192 or T * (2 * rz + 1) * body_ops > 3000:
+    if window > 192 or T * (2 * rz + 1) * body_ops > 2000:
         return {}
+    if ndim == 1:
+        below = 2048 if quotients and fp64 and T <= 3 else 0
+    elif quotients and fp64 and (r > 1 or T <= 3):
+        return {}
+    elif r <= 1:
+        below = 0 if not quotients else 10240 if fp64 else 4096
+    elif r == 2 and num_loads <= 9 and not quotients:
+        below = (0 if T <= 4 else 2048) if fp64 else (0 if T == 2 else 4096)
+    else:
+        below = 10240 if fp64 else 16384 if T == 2 else 8192
     # the strip's stored columns: at least half of the 32 lanes' points
     pad = -(-T * rx // vec) * vec
-    return {"register_chain": vec} if 2 * (32 * vec - pad - T * rx) >= 32 * vec else {}
+    if 2 * (32 * vec - pad - T * rx) < 32 * vec:
+        return {}
+    return {"register_chain": vec, "ring_below": below}
 
 
 def _rpy_keeps_registers(stencil_fn, plan, stencil_halo, halo_widths, dtype, dtype_bytes,
@@ -708,12 +767,13 @@ def compile(stencil_fn, domain: tuple[int, ...] | None = None, hw=None,
         hints["occupancy"] = occupancy
     if T > 1 and layout != "bricked":
         if kernel_hints and "register_chain" in kernel_hints:
-            for k in ("register_chain", "chain_rows", "chain_warps"):
+            for k in ("register_chain", "chain_rows", "chain_warps", "ring_below"):
                 if k in kernel_hints:
                     hints[k] = int(kernel_hints[k])
         elif tile_sizes is None and not kernel_hints and occupancy is None:
             hints.update(register_chain_plan(stencil_halo, dtype_bytes, num_inputs, T,
-                                             analysis.get("body_ops", 0), _side_planes(clone)))
+                                             analysis.get("body_ops", 0), _side_planes(clone),
+                                             num_loads, _quotients(clone)))
 
     boundary_spec = None
     if getattr(stencil_fn, "_boundary", None) is not None:

@@ -122,6 +122,7 @@ def library() -> ctypes.CDLL:
         lib.csd_module_unload.argtypes = [P]
         lib.csd_kernel_get.argtypes = [P, cp, ctypes.POINTER(P)]
         lib.csd_kernel_describe.argtypes = [P, ctypes.POINTER(KernelDesc)]
+        lib.csd_kernel_ring.argtypes = [P, ctypes.POINTER(P), ctypes.POINTER(ctypes.c_longlong)]
         lib.csd_kernel_resources.argtypes = [P, ctypes.POINTER(ctypes.c_int),
                                              ctypes.POINTER(ctypes.c_int),
                                              ctypes.POINTER(ctypes.c_int)]
@@ -284,6 +285,28 @@ class NativeKernel:
         d = KernelDesc()
         check(library().csd_kernel_describe(handle, ctypes.byref(d)))
         self.desc = d.as_dict()
+
+    def tile_rows(self, shape, halo) -> int:
+        """Rows of this kernel's tiles in an array of ``shape``: tiles across
+        its interior, times the rows (3-D: planes) of each."""
+        n = [s - 2 * h for s, h in zip(shape, halo)]
+        across = -(-n[-1] // self.desc["tile_x"])
+        if len(n) == 3:
+            across *= -(-n[1] // self.desc["tile_y"])
+        return across * (n[0] if len(n) > 1 else 1)
+
+    def batch_form(self, tile_rows: int) -> "NativeKernel":
+        """The form of this kernel for a batch of ``tile_rows`` in all: the
+        ring form of a register chain that has one, but for 3-D batches of
+        sixteen times the rows from which a launch alone takes the chain.
+        A batch's items are 16 rows, which favours the rings: 25 points FP64
+        T=3, 16 grids of 1026^2, rings 426 us, registers 624; 7 points FP64 T=2,
+        six of 32^3 25 and 41, six of 96^3 (6800 tile rows) 92 and 66."""
+        ring, below = ctypes.c_void_p(), ctypes.c_longlong()
+        check(library().csd_kernel_ring(self.handle, ctypes.byref(ring), ctypes.byref(below)))
+        if not ring.value or (self.desc["ndim"] == 3 and tile_rows >= 16 * below.value):
+            return self
+        return NativeKernel(self.name, ring)
 
     def resources(self) -> dict:
         regs, local, blocks = ctypes.c_int(), ctypes.c_int(), ctypes.c_int()

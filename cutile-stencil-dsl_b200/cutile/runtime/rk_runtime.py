@@ -165,7 +165,11 @@ class BatchLaunch:
                  bc_value: float = 0.0):
         import torch
 
-        self.kernel = kernel
+        form = kernel.batch_form(sum(kernel.tile_rows(g["inputs"][0].shape, halo)
+                                     for g in per_grid))
+        if form is not kernel and zchunk == batch_zchunk(kernel):
+            zchunk = batch_zchunk(form)      # the usual items of the form that runs
+        self.kernel = kernel = form
         gsz = native.grid_size()
         n = len(per_grid)
         host = (ctypes.c_ubyte * (gsz * n))()

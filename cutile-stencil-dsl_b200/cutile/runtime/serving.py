@@ -209,7 +209,8 @@ class StencilServer:
             if prog.spec["inputs"] != k.nstate or prog.spec["outputs"] != 1:
                 raise ValueError(f"kind {kind!r}: the stencil must read {k.nstate} field(s) and "
                                  f"write one")
-            kern = prog.kernel("main")
+            # (which solves will share a batch is not known: the form for small ones)
+            kern = prog.kernel("main").batch_form(0)
             p = (prog, kern, batch_zchunk(kern))
             self._progs[key] = p
         return p

@@ -123,6 +123,14 @@ int csd_kernel_describe(const csd_kernel* k, csd_kernel_desc* out);
  * (runtime/regcheck.py:136-212) with driver attributes. */
 int csd_kernel_resources(csd_kernel* k, int* regs, int* local_bytes, int* blocks_per_sm);
 
+/* The ring form of a register chain (`<name>_ring`, the same steps staged in
+ * shared memory), or null: csd_launch takes it for arrays of fewer than
+ * `*below` rows of the chain's tiles (tiles across X and Y, times the rows of
+ * dim 0; a quarter where rows are not aligned), unless opts ask for items
+ * (`zchunk`) or a copy path.  A batch keeps the kernel that it is given:
+ * callers look the ring form up here. */
+int csd_kernel_ring(const csd_kernel* k, csd_kernel** ring, long long* below);
+
 /* One stencil pass: read `in[0..n_in)`, write the interior of
  * `out[0..n_out)`.  Equivalent of `launch_<name>(inputs..., outputs...)`
  * (stencil_to_target.py:677-843): `temporal` steps per call for chained

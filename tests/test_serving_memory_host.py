@@ -6,7 +6,6 @@ import weakref
 from types import SimpleNamespace
 
 import pytest
-import torch
 
 from cutile.runtime import native
 from cutile.runtime.serving import SolveKind, SolveRequest, StencilServer, _Active
@@ -26,6 +25,8 @@ class CountingServer(StencilServer):
         super().__init__(KINDS, budget_bytes=budget, device="cpu")
         self.fields = weakref.WeakSet()
         self.peak = 0
+        import torch
+
         self._pool = torch.zeros(1, dtype=torch.uint8)
 
     def live(self):
@@ -67,6 +68,8 @@ class CountingServer(StencilServer):
 @pytest.fixture
 def launches(monkeypatch):
     """csd_launch_batch as a list of its calls; no pinned memory."""
+    import torch
+
     calls = []
 
     def launch_batch(handle, pool, starts, count, items, opts, stream):
