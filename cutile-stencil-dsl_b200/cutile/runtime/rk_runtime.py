@@ -210,8 +210,17 @@ def batch_zchunk(kernel: native.NativeKernel) -> int:
     bodies (kernels whose default asks for several items per resident
     block), long ones for memory-bound bodies.  Measured on the 256-grid
     shallow-water batch (8-row steps): 32-row items 130 solves/s, 16-row 124,
-    64-row 128, 8-row 107."""
+    64-row 128, 8-row 107.
+
+    A register chain (no ring slots) walks 2 T rz + T rows before an item's
+    first one, so its items need more of them; how many depends on the batch,
+    and 16 were never worse than the rings' items: heat FP64 T=5, rings / 4 / 16
+    / 32 rows: 6 grids of 258^2 45 / 18 / 14 / 17 us, 16 of 1026^2 693 / 291 /
+    121 / 97 (the split of a launch alone, 12 rows for each grid, 122; 64-row
+    items on 6 grids of 64^2 25 against 8)."""
     d = kernel.desc
+    if d["nslot"] == 0:
+        return 16
     return 4 * d["rows"] if d["zchunk"] < 0 else 64
 
 
