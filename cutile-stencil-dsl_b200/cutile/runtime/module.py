@@ -139,7 +139,8 @@ class StencilProgram:
 
         self._check(list(inputs), "reduction")
         if out is None:
-            out = torch.zeros((), dtype=torch.float64, device=inputs[0].device)
+            with native.on_stream(stream):
+                out = torch.zeros((), dtype=torch.float64, device=inputs[0].device)
         native.launch(self.kernel("main"), inputs, [], self.spec["halo"], stream,
                       scalars=self.scalar_values(scalars), red=out)
         return out
@@ -236,11 +237,12 @@ class StencilProgram:
         bs = self._brick(brick_size)
         self._check(list(inputs) + list(outputs), "stencil")
         shape = tuple(inputs[0].shape)
-        ins = [native.to_bricks(t.contiguous(), bs, stream) for t in inputs]
-        outs = [_zeros(native.bricked_shape(shape, bs), o) for o in outputs]
-        self.launch_on_bricks(ins, outs, shape, stream, scalars=scalars)
-        for o, ob in zip(outputs, outs):
-            native.from_bricks(ob, shape, bs, out=o, stream=stream)
+        with native.on_stream(stream):      # the bricked copies are this stream's
+            ins = [native.to_bricks(t.contiguous(), bs, stream) for t in inputs]
+            outs = [_zeros(native.bricked_shape(shape, bs), o) for o in outputs]
+            self.launch_on_bricks(ins, outs, shape, stream, scalars=scalars)
+            for o, ob in zip(outputs, outs):
+                native.from_bricks(ob, shape, bs, out=o, stream=stream)
 
     def apply_boundary(self, u, stream=None) -> None:
         """``apply_boundary_<name>(u)``: fill the halo of ``u`` in place."""

@@ -612,7 +612,8 @@ def to_bricks(flat, brick: int, stream=None):
     """Device bricked copy of the C-contiguous device array ``flat``."""
     import torch
 
-    out = torch.empty(bricked_shape(flat.shape, brick), dtype=flat.dtype, device=flat.device)
+    with on_stream(stream):
+        out = torch.empty(bricked_shape(flat.shape, brick), dtype=flat.dtype, device=flat.device)
     f = field_of(flat)
     check(library().csd_to_bricks(ctypes.byref(f), int(brick), ctypes.c_void_p(out.data_ptr()),
                                   ctypes.c_void_p(stream_handle(stream))))
@@ -629,7 +630,8 @@ def from_bricks(bricked, shape, brick: int, out=None, stream=None):
     if not bricked.is_contiguous():
         raise ValueError("bricked array must be contiguous")
     if out is None:
-        out = torch.empty(shape, dtype=bricked.dtype, device=bricked.device)
+        with on_stream(stream):
+            out = torch.empty(shape, dtype=bricked.dtype, device=bricked.device)
     f = field_of(out)
     check(library().csd_from_bricks(ctypes.c_void_p(bricked.data_ptr()), int(brick),
                                     ctypes.byref(f), ctypes.c_void_p(stream_handle(stream))))
