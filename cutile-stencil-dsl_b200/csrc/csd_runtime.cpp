@@ -349,6 +349,7 @@ struct csd_kernel {
   CUfunction direct = nullptr;
   csd_kernel_desc direct_desc;
   int direct_blocks_per_sm = 0;
+  unsigned direct_rewrites = 0;   // inputs (bit f) that may be outputs too
   // a register chain's ring form, the faster one on arrays of fewer than
   // ring_below rows of the chain's tiles (csd_launch), when its module has one
   csd_kernel* ring = nullptr;
@@ -493,8 +494,13 @@ int csd_kernel_get(csd_module* m, const char* name, csd_kernel** out) {
       k->direct_desc.magic == CSD_DESC_MAGIC &&
       d.cuOccupancyMaxActiveBlocksPerMultiprocessor(&k->direct_blocks_per_sm, direct,
                                                     k->direct_desc.threads, 0) == 0 &&
-      k->direct_blocks_per_sm > 0)
+      k->direct_blocks_per_sm > 0) {
     k->direct = direct;
+    unsigned mask = 0;
+    if (d.cuModuleGetGlobal(&dp, &sz, m->mod, (n + "_direct_rewrites").c_str()) == 0 &&
+        sz == sizeof(mask) && d.cuMemcpyDtoH(&mask, dp, sizeof(mask)) == 0)
+      k->direct_rewrites = mask;
+  }
   long long below = 0;
   if (d.cuModuleGetGlobal(&dp, &sz, m->mod, (n + "_ring_below").c_str()) == 0 &&
       sz == sizeof(below) && d.cuMemcpyDtoH(&below, dp, sizeof(below)) == 0 && below > 0) {
@@ -730,6 +736,16 @@ static int item_blocks(const csd_kernel_desc& D, int items) {
   return (int)(((long long)items + per - 1) / per);
 }
 
+// Whether an output is an input that the kernel's direct form loads as
+// read-only data.
+static bool overwrites(const csd_kernel* k, const csd_field* in, int n_in, const csd_field* out,
+                       int n_out) {
+  for (int i = 0; i < n_in; ++i)
+    for (int j = 0; j < n_out; ++j)
+      if (in[i].ptr == out[j].ptr && !(k->direct_rewrites >> i & 1)) return true;
+  return false;
+}
+
 // `direct_ok`: an automatic choice may fall on the kernel's direct form (its
 // descriptor suits that form only).
 static int build_grid(csd_kernel* k, const csd_field* in, int n_in, const csd_field* out,
@@ -810,7 +826,9 @@ static int build_grid(csd_kernel* k, const csd_field* in, int n_in, const csd_fi
   for (int i = 0; i < n_in; ++i) tma_ok = tma_ok && (reinterpret_cast<uintptr_t>(in[i].ptr) % 16 == 0);
   int loader = o.loader;
   if (loader < 0 || loader > 1) {   // any other value: automatic
-    loader = tma_ok ? CSD_LOADER_TMA : direct_ok && k->direct ? kLoaderDirect : CSD_LOADER_LDG;
+    loader = tma_ok ? CSD_LOADER_TMA
+             : direct_ok && k->direct && !overwrites(k, in, n_in, out, n_out) ? kLoaderDirect
+                                                                              : CSD_LOADER_LDG;
     if (loader == kLoaderDirect) D = k->direct_desc;
   }
   if (loader == CSD_LOADER_TMA && !tma_ok)

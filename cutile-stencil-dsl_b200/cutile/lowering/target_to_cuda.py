@@ -438,6 +438,8 @@ def _direct_members(kernel: KernelOp) -> list:
         _table("grp_f", "int q", by_grp(lambda f, dy, hi: f)),
         _table("grp_dy", "int q", by_grp(lambda f, dy, hi: dy)),
         _table("grp_hi", "int q", by_grp(lambda f, dy, hi: hi)),
+        f"__host__ __device__ static constexpr bool rewritten(int f) "
+        f"{{ return {engine_params(kernel)['REWRITTEN']} >> f & 1; }}",
     ]
 
 
@@ -456,6 +458,8 @@ def _emit_direct(kernel: KernelOp) -> list:
         f"  csd::direct_step<{c}, Body_{name}_direct>(p);",
         "}",
         _descriptor(f"{name}_direct_desc", c, p, 0, min_blocks, 0),
+        *([f'extern "C" __device__ const unsigned {name}_direct_rewrites = {p["REWRITTEN"]};']
+          if p["REWRITTEN"] else []),
         "",
     ]
 
@@ -525,6 +529,8 @@ def engine_params(kernel: KernelOp, ring: bool = False) -> dict:
         "BRICK": _brick_code(kernel, ndim),
         "RPY": int(hints.get("chain_rows", 0) or hints.get("rpy", 1)),
         "CHAIN_WARPS": int(hints.get("chain_warps", 4)),   # warps per block of a register chain
+        # inputs (bit f: field f) that a launch may give as outputs too
+        "REWRITTEN": int(hints.get("rewritten", 0)),
         "OCCUPANCY": int(hints.get("occupancy", 0)),   # a caller's blocks per SM (0: none)
         # points per lane of a register chain (0: the ring engine)
         "CHAIN": int(hints.get("register_chain", 0)),

@@ -1053,12 +1053,16 @@ def build_variants(stencil_fn, variants: dict, *, dtype: str | None = None,
     first = True
     for kname, opts in variants.items():
         opts = dict(opts)
-        extra_in = 0
+        extra_in, rewritten = 0, []
         if opts.get("rk") is not None:
             rk = opts["rk"]
             m = _yields(ir)
-            extra_in = ((m if rk["a"] != 0.0 and not rk.get("same_base") else 0)
-                        + (m if rk.get("w") is not None else 0))
+            for role, present in (("base", rk["a"] != 0.0 and not rk.get("same_base")),
+                                  ("acc", rk.get("w") is not None)):
+                if present:
+                    if role in rk.get("rewrites", ()):
+                        rewritten += range(n_fields + extra_in, n_fields + extra_in + m)
+                    extra_in += m
         plan = default_engine_plan(len(stencil_halo), num_loads, dtype_bytes, stencil_halo,
                                    n_fields + extra_in, _yields(ir))
         bmode = opts.pop("boundary_mode", "none")
@@ -1073,8 +1077,11 @@ def build_variants(stencil_fn, variants: dict, *, dtype: str | None = None,
         plan = fitted(plan)
         verify_engine_plan(clone, plan, stencil_halo, dtype_bytes, n_fields + extra_in,
                            periodic=bmode == "periodic")
+        hints = plan.hints()
+        if rewritten:
+            hints["rewritten"] = sum(1 << f for f in rewritten)
         target = lower_to_target_ir(ir.clone(), plan.tile_sizes(), tuple(halo_widths),
-                                    kernel_hints=plan.hints(), dtype=dtype, name=kname,
+                                    kernel_hints=hints, dtype=dtype, name=kname,
                                     boundary_spec=bspec, boundary_mode=bmode, **opts)
         parts.append(emit_cuda(target, preamble=first))
         first = False

@@ -101,8 +101,12 @@ class RKIntegrator:
 
         variants = {}
         name = self.stencil_fn._fn.__name__
-        for k, (a, b, c, w, base, stage, _acc, _out) in enumerate(_METHODS[self.method]):
-            opts = {"rk": {"a": a, "b": b, "c": c, "w": w, "same_base": base == stage}}
+        for k, (a, b, c, w, base, stage, acc, out) in enumerate(_METHODS[self.method]):
+            opts = {"rk": {"a": a, "b": b, "c": c, "w": w, "same_base": base == stage,
+                           # inputs that the stage also writes, point by point
+                           "rewrites": [n for n, hit in (("base", out == base),
+                                                         ("acc", w is not None and acc == "acc"))
+                                        if hit]}}
             if boundary is not None:
                 opts["boundary_mode"] = boundary if isinstance(boundary, str) else boundary["type"]
             variants[f"{name}_{self.method}_s{k}"] = opts
