@@ -461,9 +461,11 @@ def launch(kernel, inputs, outputs, halo, stream=None, *, plans: LaunchPlans | N
         try:
             import torch
 
-            # (the type stands for the checks that ask for torch tensors)
+            # (types stand for the checks that ask for torch tensors, and for an
+            # option's own: 1.0 == 1, but is no number of rows)
             key = (kind, torch.cuda.current_device(), len(inputs), len(scalars),
-                   tuple(kw.items()),
+                   tuple([(k, type(v), v, tuple(map(type, v)) if type(v) is tuple else None)
+                          for k, v in kw.items()]),
                    tuple([(type(t), t.dtype, t.is_cuda, t.shape, t.stride())
                           for t in (*inputs, *outputs)]))
             plan = plans.by_kind.get(key)
