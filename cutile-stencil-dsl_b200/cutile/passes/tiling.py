@@ -153,6 +153,13 @@ class EnginePlan:
     occupancy: int = 0         # explicit min_blocks request (0: fit_plan chooses)
     waves: int = 0             # auto zchunk: work items per resident block (0: fit_plan chooses)
     rpy: int = 1               # Y rows per thread (3-D, single step): strips shared by rows
+    # a register chain over this plan's rings (launcher.register_chain_plan): points per
+    # lane (0: none), rows per thread and warps per block in 3-D, and the size under
+    # which a launch takes the rings
+    register_chain: int = 0
+    chain_rows: int = 0
+    chain_warps: int = 0
+    ring_below: int = 0
 
     @property
     def units_per_step(self) -> int:
@@ -174,6 +181,11 @@ class EnginePlan:
              "zchunk": self.zchunk, "min_blocks": self.min_blocks, "waves": self.waves}
         if self.rpy != 1:
             h["rpy"] = self.rpy
+        if self.register_chain:
+            h["register_chain"] = self.register_chain
+            if self.chain_rows:
+                h["chain_rows"], h["chain_warps"] = self.chain_rows, self.chain_warps
+            h["ring_below"] = self.ring_below
         return h
 
 

@@ -4,7 +4,8 @@ The reference (runtime/autotune.py:88-309) times cuTile tile shapes and
 temporal depths on the GPU and caches the winner per stencil name and GPU.
 Here the search is over the engine plan -- rows per streaming step, tile
 (Y, X), threads, chunks in flight, work items per resident block, temporal
-depth -- and the cache is keyed by what decides the best plan: the stencil's
+depth, and for depths above one the register chain that compile() would use --
+and the cache is keyed by what decides the best plan: the stencil's
 footprint (per-dimension radius, distinct loads, fields in and out), the
 dtype, the dimensionality and the grid-size class (log2 of the interior
 points), plus the GPU name.  Every candidate goes through ``fit_plan`` (box,
@@ -22,7 +23,7 @@ import os
 import threading
 from dataclasses import asdict, dataclass, field, replace
 
-_CACHE_VERSION = "b200-v1"
+_CACHE_VERSION = "b200-v2"
 _lock = threading.Lock()
 
 
@@ -45,12 +46,14 @@ def cache_path() -> str:
 
 
 def _footprint(stencil_fn, dtype_bytes: int):
-    from cutile.runtime.launcher import Pipeline, _analysis_of, _num_inputs, _yields
+    from cutile.runtime.launcher import (Pipeline, _analysis_of, _num_inputs, _quotients,
+                                         _side_planes, _yields)
 
     clone = stencil_fn._ir.clone()
-    Pipeline.single_gpu(dtype_bytes=dtype_bytes, max_temporal_steps=1).run(clone)
-    halo, _t, _T, analysis, _o, num_loads = _analysis_of(clone)
-    return {"radius": list(halo), "loads": num_loads, "inputs": _num_inputs(stencil_fn._ir),
+    Pipeline.single_gpu(dtype_bytes=dtype_bytes, max_temporal_steps=8).run(clone)
+    halo, _t, depth, analysis, _o, num_loads = _analysis_of(clone)
+    return {"depth": depth, "side_planes": _side_planes(clone), "quotients": _quotients(clone),
+            "radius": list(halo), "loads": num_loads, "inputs": _num_inputs(stencil_fn._ir),
             "outputs": _yields(stencil_fn._ir), "body_ops": analysis.get("body_ops", 0)}
 
 
@@ -60,7 +63,24 @@ def cache_key(fp: dict, dtype: str, domain, gpu: str) -> str:
         pts *= int(n)
     size_class = int(round(math.log2(max(1, pts))))
     return (f"{_CACHE_VERSION}|{gpu}|{dtype}|nd{len(domain)}|r{fp['radius']}|l{fp['loads']}|"
-            f"i{fp['inputs']}o{fp['outputs']}|b{fp['body_ops']}|s{size_class}")
+            f"i{fp['inputs']}o{fp['outputs']}|b{fp['body_ops']}|d{fp.get('depth', 1)}|"
+            f"y{fp.get('side_planes', 0)}|q{int(fp.get('quotients', False))}|s{size_class}")
+
+
+def _depths(ndim: int) -> tuple:
+    """Temporal depths that single-field bodies are timed at."""
+    return {3: (1, 2), 2: (1, 2, 4), 1: (1, 2, 4, 8)}[ndim]
+
+
+def chain_hints(fp: dict, ndim: int, dtype_bytes: int) -> dict:
+    """depth -> hints of the register chain that compile() takes there ({}: its
+    rings), for the depths to time and compile()'s own depth."""
+    from cutile.runtime.launcher import register_chain_plan
+
+    return {T: register_chain_plan(tuple(fp["radius"]), dtype_bytes, fp["inputs"], T,
+                                   fp["body_ops"], fp["side_planes"], fp["loads"],
+                                   fp["quotients"])
+            for T in sorted({*_depths(ndim), fp["depth"]}) if T > 1}
 
 
 def _load(key: str):
@@ -89,15 +109,19 @@ def _save(key: str, entry: dict) -> None:
 
 def candidates(ndim: int, dtype_bytes: int, radius, num_inputs: int, num_loads: int,
                body_ops: int, single_field: bool, max_candidates: int = 30,
-               num_outputs: int = 1) -> list:
-    """Distinct fitted plans around the default one, most promising first."""
+               num_outputs: int = 1, chains: dict | None = None) -> list:
+    """Distinct fitted plans around the default one, most promising first;
+    ``chains`` (``chain_hints``) adds compile()'s own plan of each depth."""
     from cutile.passes.tiling import EnginePlan, default_engine_plan, fit_plan
+    from cutile.runtime.launcher import chain_tile
 
     vec = 16 // dtype_bytes
     base = default_engine_plan(ndim, num_loads, dtype_bytes, tuple(radius), num_inputs,
                                num_outputs)
     raw = [base]
-    depths = (1, 2) if single_field else (1,)
+    raw += [replace(base, temporal=T, rpy=1, **chain_tile(ndim, dtype_bytes, T), **h)
+            for T, h in (chains or {}).items()]
+    depths = _depths(ndim) if single_field else (1,)
     if ndim == 3:
         shapes = [(1, 4, 128), (1, 8, 128), (1, 2, 128), (1, 16, 64), (1, 8, 64), (1, 4, 64),
                   (2, 4, 128), (1, 16, 128), (1, 32, 32)]
@@ -110,13 +134,13 @@ def candidates(ndim: int, dtype_bytes: int, radius, num_inputs: int, num_loads: 
         for rows in (4, 8, 16):
             for tx in (64, 128):
                 for nt in (128, 256):
-                    for T in (depths + ((4,) if single_field else ())):
+                    for T in depths:
                         raw.append(EnginePlan(2, rows=rows, tile_y=1, tile_x=tx, vec=vec,
                                               threads=nt, stages=1, zchunk=0, temporal=T))
     else:
         for tx in (64, 128):
             for nt in (64, 128, 256):
-                for T in (depths + ((4, 8) if single_field else ())):
+                for T in depths:
                     raw.append(EnginePlan(1, rows=1, tile_y=1, tile_x=tx, vec=vec, threads=nt,
                                           stages=0, zchunk=0, temporal=T))
     out, seen = [], set()
@@ -127,7 +151,8 @@ def candidates(ndim: int, dtype_bytes: int, radius, num_inputs: int, num_loads: 
             continue
         if f.rows < radius[0] if ndim > 1 else False:
             continue
-        key = (f.rows, f.tile_y, f.tile_x, f.threads, f.stages, f.temporal, f.min_blocks, f.rpy)
+        key = (f.rows, f.tile_y, f.tile_x, f.threads, f.stages, f.temporal, f.min_blocks, f.rpy,
+               f.register_chain)
         if key in seen:
             continue
         seen.add(key)
@@ -139,8 +164,12 @@ def probe_hints(p) -> dict:
     """The kernel hints that make ``compile(tile_sizes=p.tile_sizes(), ...)``
     build exactly the candidate plan ``p`` (rows per thread included), so the
     plan that is timed is the plan that is returned."""
-    return {"threads": p.threads, "stages": p.stages, "zchunk": p.zchunk,
-            "min_blocks": p.min_blocks, "waves": p.waves, "rows_per_thread": p.rpy}
+    h = {"threads": p.threads, "stages": p.stages, "zchunk": p.zchunk,
+         "min_blocks": p.min_blocks, "waves": p.waves, "rows_per_thread": p.rpy}
+    for key in ("register_chain", "chain_rows", "chain_warps", "ring_below"):
+        if p.register_chain and key in p.hints():
+            h[key] = p.hints()[key]
+    return h
 
 
 def _gpu_name() -> str:
@@ -154,10 +183,12 @@ def _gpu_name() -> str:
 
 def autotune(stencil_fn, domain=None, hw=None, *, dtype: str | None = None,
              max_candidates: int = 30, warmup: int = 3, iters: int = 10,
-             verbose: bool = False, use_cache: bool = True) -> AutotuneResult:
+             verbose: bool = False, use_cache: bool = True,
+             chains: bool = True) -> AutotuneResult:
     """Time candidate plans of ``stencil_fn`` on a synthetic ``domain``
     (interior extents) and return the fastest; cached per footprint, dtype,
-    dimensionality, size class and GPU."""
+    dimensionality, size class and GPU.  ``chains=False`` leaves register
+    chains out (layouts that have none)."""
     import numpy as np
     import torch
 
@@ -175,7 +206,7 @@ def autotune(stencil_fn, domain=None, hw=None, *, dtype: str | None = None,
     fp = _footprint(stencil_fn, dtype_bytes)
     ndim = len(domain)
     gpu = _gpu_name()
-    key = cache_key(fp, dtype, domain, gpu)
+    key = cache_key(fp, dtype, domain, gpu) + ("" if chains else "|rings")
     if use_cache:
         hit = _load(key)
         if hit is not None:
@@ -187,7 +218,8 @@ def autotune(stencil_fn, domain=None, hw=None, *, dtype: str | None = None,
                                   hit.get("candidates", 0))
     single = fp["inputs"] == 1 and fp["outputs"] == 1
     plans = candidates(ndim, dtype_bytes, fp["radius"], fp["inputs"], fp["loads"],
-                       fp["body_ops"], single, max_candidates, fp["outputs"])
+                       fp["body_ops"], single, max_candidates, fp["outputs"],
+                       chain_hints(fp, ndim, dtype_bytes) if single and chains else None)
     if not torch.cuda.is_available():
         raise RuntimeError("autotune times candidates on the GPU; no CUDA device is visible")
     pts = 1

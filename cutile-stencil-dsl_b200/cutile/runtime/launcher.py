@@ -490,6 +490,13 @@ def chain_tile_2d(dtype_bytes: int, T: int) -> dict:
     return dict(rows=4, tile_x=128, threads=256)
 
 
+def chain_tile(ndim: int, dtype_bytes: int, T: int) -> dict:
+    """What a chain of T > 1 steps changes in the default plan."""
+    if ndim == 3:
+        return dict(rows=1, **chain_tile_3d(dtype_bytes, T))
+    return chain_tile_2d(dtype_bytes, T) if ndim == 2 else {}
+
+
 def _side_planes(ir) -> int:
     """Planes of the rows beside a thread's own that a 3-D register chain
     holds: from the leading plane to the last one the body reads off centre."""
@@ -717,12 +724,13 @@ def compile(stencil_fn, domain: tuple[int, ...] | None = None, hw=None,
     plan = default_engine_plan(len(stencil_halo), num_loads, dtype_bytes, stencil_halo, num_inputs,
                                _yields(ir))
     resources = None
+    tuned = None
     if autotune and domain is not None:
         from cutile.runtime.autotune import autotune as _autotune
 
-        res = _autotune(stencil_fn, domain, hw=hw, dtype=dtype)
+        res = _autotune(stencil_fn, domain, hw=hw, dtype=dtype, chains=layout != "bricked")
         if res.plan is not None:
-            plan = res.plan
+            plan = tuned = res.plan
         T = res.temporal_steps
     if kahan:
         num_inputs += 1  # the compensation field
@@ -739,18 +747,21 @@ def compile(stencil_fn, domain: tuple[int, ...] | None = None, hw=None,
         # (stencil_to_target.py:796-800), so a multi-field stencil cannot run
         # blocked there either; it advances one step per launch.
         T = 1
-    plan = replace(plan, temporal=T, rpy=plan.rpy if T == 1 else 1)
+    # a tuned plan is compiled as it was timed, unless the call asks for more
+    as_timed = (tuned is not None and tuned.temporal == T and layout != "bricked" and not kahan
+                and tile_sizes is None and not kernel_hints and occupancy is None)
+    if not as_timed:
+        plan = replace(plan, temporal=T, rpy=plan.rpy if T == 1 else 1, register_chain=0,
+                       chain_rows=0, chain_warps=0, ring_below=0)
     hinted_rpy = bool(kernel_hints) and ("rows_per_thread" in kernel_hints or "rpy" in kernel_hints)
-    if plan.rpy > 1 and tile_sizes is None and not hinted_rpy and not _rpy_keeps_registers(
+    if plan.rpy > 1 and tile_sizes is None and not hinted_rpy and not as_timed and not _rpy_keeps_registers(
             stencil_fn, plan, stencil_halo, halo_widths, dtype, dtype_bytes, num_inputs, T,
             analysis.get("body_ops", 0), kahan):
         # the default rows-per-thread plan would spill this body's strips:
         # one row per thread over the wide tile instead
         plan = replace(plan, rpy=1, rows=1, tile_y=4, tile_x=64)
-    if T > 1 and len(stencil_halo) == 3 and tile_sizes is None and not plan.rpy > 1:
-        plan = replace(plan, rows=1, **chain_tile_3d(dtype_bytes, T))
-    elif T > 1 and len(stencil_halo) == 2 and tile_sizes is None:
-        plan = replace(plan, **chain_tile_2d(dtype_bytes, T))
+    if T > 1 and tile_sizes is None and not as_timed and not plan.rpy > 1:
+        plan = replace(plan, **chain_tile(len(stencil_halo), dtype_bytes, T))
     if layout == "bricked" and len(stencil_halo) == 3 and tile_sizes is None:
         # one Z row per chunk, so that the bricked kernel can stage bricks
         # with tensor copies (target_to_cuda.brick_tma_eligible)
@@ -765,7 +776,7 @@ def compile(stencil_fn, domain: tuple[int, ...] | None = None, hw=None,
     hints = plan.hints()
     if occupancy is not None:
         hints["occupancy"] = occupancy
-    if T > 1 and layout != "bricked":
+    if T > 1 and layout != "bricked" and not as_timed:
         if kernel_hints and "register_chain" in kernel_hints:
             for k in ("register_chain", "chain_rows", "chain_warps", "ring_below"):
                 if k in kernel_hints:
