@@ -14,6 +14,7 @@
 #include <sys/stat.h>
 #include <unistd.h>
 
+#include <atomic>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
@@ -77,6 +78,7 @@ struct Driver {
   CUresult (*cuGetErrorString)(CUresult, const char**);
   CUresult (*cuCtxSynchronize)(void);
   CUresult (*cuCtxGetId)(CUcontext, unsigned long long*);  // optional (driver >= 12.0)
+  CUresult (*cuStreamIsCapturing)(CUstream, int*);
 };
 
 static thread_local std::string g_last_error;
@@ -135,6 +137,7 @@ static void load_driver(Driver& d) {
   CSD_SYM(cuTensorMapEncodeTiled, "cuTensorMapEncodeTiled");
   CSD_SYM(cuGetErrorString, "cuGetErrorString");
   CSD_SYM(cuCtxSynchronize, "cuCtxSynchronize");
+  CSD_SYM(cuStreamIsCapturing, "cuStreamIsCapturing");
 #undef CSD_SYM
   d.cuCtxGetId = reinterpret_cast<decltype(d.cuCtxGetId)>(dlsym(h, "cuCtxGetId"));
   if (d.cuInit(0) != 0) {
@@ -345,15 +348,22 @@ struct csd_kernel {
   CUfunction fn[2] = {nullptr, nullptr};  // [CSD_LOADER_TMA], [CSD_LOADER_LDG]
   csd_kernel_desc desc;
   int blocks_per_sm[2] = {0, 0};
-  // the kernel's direct form (engine.cuh DirectCfg), when its module has one
-  CUfunction direct = nullptr;
+  // Forms (csd.h), null until a module that has them is loaded; the pointers
+  // are set last, so that a launch on another thread sees a form whole.
+  // The direct form (engine.cuh DirectCfg):
+  std::atomic<CUfunction> direct{nullptr};
   csd_kernel_desc direct_desc;
   int direct_blocks_per_sm = 0;
   unsigned direct_rewrites = 0;   // inputs (bit f) that may be outputs too
   // a register chain's ring form, the faster one on arrays of fewer than
-  // ring_below rows of the chain's tiles (csd_launch), when its module has one
-  csd_kernel* ring = nullptr;
+  // ring_below rows of the chain's tiles (csd_launch):
+  std::atomic<csd_kernel*> ring{nullptr};
   long long ring_below = 0;
+  // the kernels that batches launch (their own in register chains):
+  std::atomic<bool> batched{false};
+  CUfunction batch_fn[2] = {nullptr, nullptr};
+  // forms (bit CSD_FORM_*) that the caller attaches when a launch wants them
+  std::atomic<unsigned> deferred{0};
   std::string name;
 };
 
@@ -438,6 +448,59 @@ int csd_module_unload(csd_module* m) {
   return CSD_OK;
 }
 
+static bool has_form(const csd_kernel* k, int form) {
+  return form == CSD_FORM_DIRECT ? k->direct != nullptr
+         : form == CSD_FORM_RING ? k->ring != nullptr
+                                 : k->batched.load();
+}
+
+// Look `form` of the kernel up in module `m`; whether it is there.
+static bool attach_form(csd_kernel* k, csd_module* m, int form) {
+  Driver& d = drv();
+  const std::string& n = k->name;
+  CUdeviceptr dp;
+  size_t sz;
+  if (form == CSD_FORM_DIRECT) {
+    CUfunction fn = nullptr;
+    if (d.cuModuleGetFunction(&fn, m->mod, (n + "_direct").c_str()) != 0 ||
+        d.cuModuleGetGlobal(&dp, &sz, m->mod, (n + "_direct_desc").c_str()) != 0 ||
+        sz != sizeof(csd_kernel_desc) ||
+        d.cuMemcpyDtoH(&k->direct_desc, dp, sizeof(csd_kernel_desc)) != 0 ||
+        k->direct_desc.magic != CSD_DESC_MAGIC ||
+        d.cuOccupancyMaxActiveBlocksPerMultiprocessor(&k->direct_blocks_per_sm, fn,
+                                                      k->direct_desc.threads, 0) != 0 ||
+        k->direct_blocks_per_sm < 1)
+      return false;
+    unsigned mask = 0;
+    if (d.cuModuleGetGlobal(&dp, &sz, m->mod, (n + "_direct_rewrites").c_str()) == 0 &&
+        sz == sizeof(mask) && d.cuMemcpyDtoH(&mask, dp, sizeof(mask)) == 0)
+      k->direct_rewrites = mask;
+    k->direct = fn;
+    return true;
+  }
+  if (form == CSD_FORM_RING) {
+    csd_kernel* ring = nullptr;
+    if (d.cuModuleGetGlobal(&dp, &sz, m->mod, (n + "_ring_desc").c_str()) != 0 ||
+        csd_kernel_get(m, (n + "_ring").c_str(), &ring) != CSD_OK)
+      return false;
+    ring->name = n;
+    k->ring = ring;
+    return true;
+  }
+  CUfunction fn[2];
+  if (d.cuModuleGetFunction(&fn[CSD_LOADER_TMA], m->mod, (n + "_batch_tma").c_str()) != 0 ||
+      d.cuModuleGetFunction(&fn[CSD_LOADER_LDG], m->mod, (n + "_batch_ldg").c_str()) != 0)
+    return false;
+  for (CUfunction f : fn)
+    if (d.cuFuncSetAttribute(f, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES_,
+                             k->desc.smem_bytes) != 0)
+      return false;
+  k->batch_fn[0] = fn[0];
+  k->batch_fn[1] = fn[1];
+  k->batched = true;
+  return true;
+}
+
 int csd_kernel_get(csd_module* m, const char* name, csd_kernel** out) {
   if (!m || !name || !out) return fail(CSD_EINVAL, "null argument");
   Driver& d = drv();
@@ -486,33 +549,36 @@ int csd_kernel_get(csd_module* m, const char* name, csd_kernel** out) {
     }
     if (k->blocks_per_sm[l] < 1) k->blocks_per_sm[l] = 1;
   }
-  CUfunction direct = nullptr;
-  if (d.cuModuleGetFunction(&direct, m->mod, (n + "_direct").c_str()) == 0 &&
-      d.cuModuleGetGlobal(&dp, &sz, m->mod, (n + "_direct_desc").c_str()) == 0 &&
-      sz == sizeof(csd_kernel_desc) &&
-      d.cuMemcpyDtoH(&k->direct_desc, dp, sizeof(csd_kernel_desc)) == 0 &&
-      k->direct_desc.magic == CSD_DESC_MAGIC &&
-      d.cuOccupancyMaxActiveBlocksPerMultiprocessor(&k->direct_blocks_per_sm, direct,
-                                                    k->direct_desc.threads, 0) == 0 &&
-      k->direct_blocks_per_sm > 0) {
-    k->direct = direct;
-    unsigned mask = 0;
-    if (d.cuModuleGetGlobal(&dp, &sz, m->mod, (n + "_direct_rewrites").c_str()) == 0 &&
-        sz == sizeof(mask) && d.cuMemcpyDtoH(&mask, dp, sizeof(mask)) == 0)
-      k->direct_rewrites = mask;
-  }
   long long below = 0;
   if (d.cuModuleGetGlobal(&dp, &sz, m->mod, (n + "_ring_below").c_str()) == 0 &&
-      sz == sizeof(below) && d.cuMemcpyDtoH(&below, dp, sizeof(below)) == 0 && below > 0) {
-    const int rc = csd_kernel_get(m, (n + "_ring").c_str(), &k->ring);
-    if (rc) {
-      delete k;
-      return rc;
-    }
-    k->ring->name = n;
+      sz == sizeof(below) && d.cuMemcpyDtoH(&below, dp, sizeof(below)) == 0)
     k->ring_below = below;
+  if (d.cuModuleGetGlobal(&dp, &sz, m->mod, (n + "_batch_apart").c_str()) != 0) {
+    k->batch_fn[0] = k->fn[0];
+    k->batch_fn[1] = k->fn[1];
+    k->batched = true;
   }
+  // (a form that does not load is as good as one that the module lacks)
+  for (int form = CSD_FORM_DIRECT; form <= CSD_FORM_BATCH; ++form) attach_form(k, m, form);
   *out = k;
+  return CSD_OK;
+}
+
+int csd_kernel_attach(csd_kernel* k, csd_module* m, int form) {
+  if (!k || !m || form < CSD_FORM_DIRECT || form > CSD_FORM_BATCH)
+    return fail(CSD_EINVAL, "bad arguments");
+  static std::mutex mu;
+  std::lock_guard<std::mutex> lock(mu);
+  if (!has_form(k, form) && !attach_form(k, m, form))
+    return fail(CSD_ENOSYM, "the module holds no form %d of kernel %s", form, k->name.c_str());
+  k->deferred &= ~(1u << form);
+  return CSD_OK;
+}
+
+int csd_kernel_defer(csd_kernel* k, int form) {
+  if (!k || (form != CSD_FORM_DIRECT && form != CSD_FORM_RING))
+    return fail(CSD_EINVAL, "bad arguments");
+  if (!has_form(k, form)) k->deferred |= 1u << form;
   return CSD_OK;
 }
 
@@ -746,11 +812,20 @@ static bool overwrites(const csd_kernel* k, const csd_field* in, int n_in, const
   return false;
 }
 
+// Whether a launch on `stream` that would take a form asks for it to be
+// attached first (a capture must not wait for a compiler or load a module).
+static bool wants(const csd_kernel* k, int form, void* stream) {
+  if (!(k->deferred >> form & 1)) return false;
+  int capturing = 0;
+  return drv().cuStreamIsCapturing(reinterpret_cast<CUstream>(stream), &capturing) == 0 &&
+         capturing == 0;
+}
+
 // `direct_ok`: an automatic choice may fall on the kernel's direct form (its
-// descriptor suits that form only).
+// descriptor suits that form only), for a launch on `stream`.
 static int build_grid(csd_kernel* k, const csd_field* in, int n_in, const csd_field* out,
                       int n_out, const csd_launch_opts& o, DeviceState* st, bool direct_ok,
-                      csd_grid* g, int* loader_out) {
+                      void* stream, csd_grid* g, int* loader_out) {
   csd_kernel_desc D = k->desc;
   if (!in || (!out && n_out > 0)) return fail(CSD_EINVAL, "null field array");
   if (D.reduce_max && !o.red)
@@ -826,9 +901,13 @@ static int build_grid(csd_kernel* k, const csd_field* in, int n_in, const csd_fi
   for (int i = 0; i < n_in; ++i) tma_ok = tma_ok && (reinterpret_cast<uintptr_t>(in[i].ptr) % 16 == 0);
   int loader = o.loader;
   if (loader < 0 || loader > 1) {   // any other value: automatic
-    loader = tma_ok ? CSD_LOADER_TMA
-             : direct_ok && k->direct && !overwrites(k, in, n_in, out, n_out) ? kLoaderDirect
-                                                                              : CSD_LOADER_LDG;
+    loader = tma_ok ? CSD_LOADER_TMA : CSD_LOADER_LDG;
+    if (!tma_ok && direct_ok && !overwrites(k, in, n_in, out, n_out)) {
+      if (k->direct)
+        loader = kLoaderDirect;
+      else if (wants(k, CSD_FORM_DIRECT, stream))
+        return fail(CSD_EDIRECT, "the direct form of kernel %s is to be attached", k->name.c_str());
+    }
     if (loader == kLoaderDirect) D = k->direct_desc;
   }
   if (loader == CSD_LOADER_TMA && !tma_ok)
@@ -943,7 +1022,8 @@ int csd_launch(csd_kernel* k, const csd_field* in, int n_in, const csd_field* ou
   memset(&p, 0, sizeof(p));
   int loader = 0;
   // a withheld input chunk needs a kernel that stages chunks
-  rc = build_grid(k, in, n_in, out, n_out, o, st, o.withhold_chunk <= 0, &p.g, &loader);
+  rc = build_grid(k, in, n_in, out, n_out, o, st, o.withhold_chunk <= 0, stream, &p.g,
+                  &loader);
   if (rc) return rc;
   // a chain's items and copies may be asked for by zchunk and loader; left to
   // the library, arrays that are small for it take the rings.  Rows that are
@@ -951,11 +1031,15 @@ int csd_launch(csd_kernel* k, const csd_field* in, int n_in, const csd_field* ou
   // rings / registers us: 257 x 259 25 / 27, 513 x 515 49 / 33, aligned 512^2
   // 25 / 33), so a quarter of the size decides there.
   const long long limit = loader == CSD_LOADER_TMA ? k->ring_below : k->ring_below / 4;
-  if (k->ring && (o.loader < 0 || o.loader > 1) && o.zchunk <= 0 && o.withhold_chunk <= 0 &&
+  if (limit > 0 && (o.loader < 0 || o.loader > 1) && o.zchunk <= 0 && o.withhold_chunk <= 0 &&
       (long long)p.g.tiles[0] * p.g.tiles[1] * p.g.interior[0] < limit) {
-    k = k->ring;
-    rc = build_grid(k, in, n_in, out, n_out, o, st, false, &p.g, &loader);
-    if (rc) return rc;
+    if (k->ring) {
+      k = k->ring;
+      rc = build_grid(k, in, n_in, out, n_out, o, st, false, stream, &p.g, &loader);
+      if (rc) return rc;
+    } else if (wants(k, CSD_FORM_RING, stream)) {
+      return fail(CSD_ERING, "the ring form of kernel %s is to be attached", k->name.c_str());
+    }
   }
   const csd_kernel_desc& D = loader == kLoaderDirect ? k->direct_desc : k->desc;
   p.err = reinterpret_cast<int*>(st->err);
@@ -966,7 +1050,7 @@ int csd_launch(csd_kernel* k, const csd_field* in, int n_in, const csd_field* ou
   if (grid > blocks) grid = blocks;
   if (grid < 1) return CSD_OK;  // nothing to do
   void* args[] = {&p};
-  CUresult r = drv().cuLaunchKernel(loader == kLoaderDirect ? k->direct : k->fn[loader],
+  CUresult r = drv().cuLaunchKernel(loader == kLoaderDirect ? k->direct.load() : k->fn[loader],
                                     (unsigned)grid, 1, 1, (unsigned)D.threads, 1, 1,
                                     (unsigned)D.smem_bytes,
                                     reinterpret_cast<CUstream>(stream), args, nullptr);
@@ -987,7 +1071,7 @@ int csd_grid_build(csd_kernel* k, const csd_field* in, int n_in, const csd_field
   rc = device_state(dev, &st);
   if (rc) return rc;
   int loader = 0;
-  rc = build_grid(k, in, n_in, out, n_out, o, st, false, g, &loader);
+  rc = build_grid(k, in, n_in, out, n_out, o, st, false, nullptr, g, &loader);
   if (rc) return rc;
   if (items) *items = g->items;
   if (loader_used) *loader_used = loader;
@@ -1017,11 +1101,13 @@ int csd_launch_batch(csd_kernel* k, const csd_grid* grids, const int* item_start
   p.timeout_ns = (opts && opts->timeout_ns) ? opts->timeout_ns : 2000000000ull;
   p.withhold = (opts && opts->withhold_chunk > 0) ? opts->withhold_chunk : 0;
   const int loader = (opts && opts->loader == CSD_LOADER_LDG) ? CSD_LOADER_LDG : CSD_LOADER_TMA;
+  if (!k->batched)
+    return fail(CSD_ENOSYM, "the batch form of kernel %s is not attached", k->name.c_str());
   int grid = (opts && opts->grid > 0) ? opts->grid : k->blocks_per_sm[loader] * st->sms;
   const int blocks = item_blocks(k->desc, total_items);
   if (grid > blocks) grid = blocks;
   void* args[] = {&p};
-  CUresult r = drv().cuLaunchKernel(k->fn[loader], (unsigned)grid, 1, 1,
+  CUresult r = drv().cuLaunchKernel(k->batch_fn[loader], (unsigned)grid, 1, 1,
                                     (unsigned)k->desc.threads, 1, 1, (unsigned)k->desc.smem_bytes,
                                     reinterpret_cast<CUstream>(stream), args, nullptr);
   if (r) return cu_fail(r, "cuLaunchKernel(batch)");

@@ -958,12 +958,11 @@ __device__ __forceinline__ void chain_items(const csd_params& p) {
   }
 }
 
-template <class C, class Body>
+// (a batch's grids are read from memory, a launch's own from its parameters:
+// kernels of their own, compiled when the first batch arrives)
+template <class C, class Body, bool BATCHED>
 __device__ __forceinline__ void register_chain(const csd_params& p) {
-  if (p.grids == nullptr)
-    chain_items<C, Body, false>(p);
-  else
-    chain_items<C, Body, true>(p);
+  chain_items<C, Body, BATCHED>(p);
 }
 
 // ---------------------------------------------------------------------------
@@ -1217,12 +1216,9 @@ __device__ __forceinline__ void plane_chain_items(const csd_params& p) {
   }
 }
 
-template <class C, class Body>
+template <class C, class Body, bool BATCHED>
 __device__ __forceinline__ void plane_chain(const csd_params& p) {
-  if (p.grids == nullptr)
-    plane_chain_items<C, Body, false>(p);
-  else
-    plane_chain_items<C, Body, true>(p);
+  plane_chain_items<C, Body, BATCHED>(p);
 }
 
 // ---------------------------------------------------------------------------

@@ -591,18 +591,35 @@ def _emit_engine(name: str, p: dict) -> list:
                        f"{p['RY']}, {p['RX']}, {nt}, {p['TEMPORAL']}, {loader}, {p['VEC']}, "
                        f"{p['RPY']}>")
         parts.append(f"typedef {cfg} Cfg_{name}_{suffix};")
-        parts.append(f'extern "C" __global__ void __launch_bounds__({nt}, {minb})')
-        parts.append(f"{name}_{suffix}(const __grid_constant__ csd_params p) {{")
-        parts.append(f"  csd::{entry}<Cfg_{name}_{suffix}, Body_{name}>(p);")
-        parts.append("}")
+        # chains have kernels of their own for batches
+        for form, infix, last in (((0, "", ", false"), (3, "batch_", ", true")) if p["CHAIN"] else
+                                  ((0, "", ""),)):
+            if p["CHAIN"]:
+                parts.append(f"#if CSD_HAS({form})")
+            parts.append(f'extern "C" __global__ void __launch_bounds__({nt}, {minb})')
+            parts.append(f"{name}_{infix}{suffix}(const __grid_constant__ csd_params p) {{")
+            parts.append(f"  csd::{entry}<Cfg_{name}_{suffix}, Body_{name}{last}>(p);")
+            parts.append("}")
+            if p["CHAIN"]:
+                parts.append("#endif")
+    if p["CHAIN"]:
+        parts += ["#if CSD_HAS(0)", f'extern "C" __device__ const int {name}_batch_apart = 1;']
     c = f"Cfg_{name}_tma"
     # both entries launch with one shared-memory size: the larger one
     smem = (f"({c}::SMEM_BYTES > Cfg_{name}_ldg::SMEM_BYTES ? {c}::SMEM_BYTES : "
             f"Cfg_{name}_ldg::SMEM_BYTES)")
     parts.append(_descriptor(f"{name}_desc", c, p, p["ZCHUNK"], p["MINB"],
                              1 if brick_tma else 0, smem))
+    if p["CHAIN"]:
+        parts.append("#endif")
     parts.append("")
     return parts
+
+
+def source_forms(source: str, name: str) -> tuple:
+    """Forms of kernel ``name`` beside its own that a generated source holds."""
+    return tuple(f for f, mark in ((1, f"{name}_direct_desc = {{"), (2, f"{name}_ring_desc = {{"),
+                                   (3, f"{name}_batch_apart = ")) if f" {mark}" in source)
 
 
 def emit_cuda(module: ModuleOp, preamble: bool = True) -> str:
@@ -612,6 +629,10 @@ def emit_cuda(module: ModuleOp, preamble: bool = True) -> str:
     if not kernels:
         raise ValueError("No KernelOp found in target IR module")
     parts = ["// Generated B200 stencil kernel(s). Do not edit.",
+             "// Forms: 0 the kernels themselves, 1 for unaligned rows, 2 rings of register",
+             "// chains, 3 batches of register chains; all of them unless CSD_FORM names one.",
+             "#ifdef CSD_FORM", "#define CSD_HAS(form) (CSD_FORM == (form))", "#else",
+             "#define CSD_HAS(form) 1", "#endif",
              '#include "csd/engine.cuh"', "",
              "__device__ __forceinline__ double csd_max(double a, double b) "
              "{ return (a != a || a > b) ? a : b; }",
@@ -627,21 +648,26 @@ def emit_cuda(module: ModuleOp, preamble: bool = True) -> str:
         name = kernel.kernel_name.data
         p = engine_params(kernel)
         parts.append(f"// expression: {kernel.expression.data}")
+        parts.append("#if CSD_HAS(0) || CSD_HAS(3)" if p["CHAIN"] else "#if CSD_HAS(0)")
         parts.append(emit_body(kernel))
         parts.append("")
         parts.extend(_emit_engine(name, p))
+        parts.append("#endif")
         if p["CHAIN"] and p["RING_BELOW"] > 0:
             # the same steps by the shared-memory rings, for smaller arrays
             q = engine_params(kernel, ring=True)
+            parts += ["#if CSD_HAS(0)", f'extern "C" __device__ const long long {name}_ring_below = '
+                      f'{p["RING_BELOW"]};', "#endif", "#if CSD_HAS(2)"]
             parts.append(emit_body(kernel, q["VEC"], "_ring"))
             parts.append("")
             parts.extend(_emit_engine(f"{name}_ring", q))
-            parts.append(f'extern "C" __device__ const long long {name}_ring_below = '
-                         f'{p["RING_BELOW"]};')
-            parts.append("")
+            parts.append("#endif")
         if direct_plan(kernel)[0]:
+            parts.append("#if CSD_HAS(1)")
             parts.extend(_emit_direct(kernel))
+            parts.append("#endif")
+        parts.append("")
     return "\n".join(parts) + "\n"
 
 
-__all__ = ["emit_cuda", "emit_body", "engine_params", "hex_literal", "brick_tma_eligible"]
+__all__ = ["emit_cuda", "source_forms", "emit_body", "engine_params", "hex_literal", "brick_tma_eligible"]

@@ -642,7 +642,7 @@ def _rpy_keeps_registers(stencil_fn, plan, stencil_halo, halo_widths, dtype, dty
                                 temporal_steps=T, kernel_hints=p.hints(), dtype=dtype,
                                 kahan=kahan)
     try:
-        _, log = native.compile_source(emit_cuda(target))
+        _, log = native.compile_source(emit_cuda(target), native.form_option(0))
     except Exception:  # noqa: BLE001 - no NVRTC here: keep the measured default
         return True
     res = parse_ptxas_log(log, f"{stencil_fn._fn.__name__}_tma")

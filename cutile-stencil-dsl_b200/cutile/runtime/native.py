@@ -20,6 +20,7 @@ LIB_PATH = PKG_DIR / "_native" / "libcsd.so"
 INCLUDE_DIR = ROOT_DIR / "csrc" / "include"
 HEADER_NAMES = ("csd/params.h", "csd/ptx.cuh", "csd/engine.cuh")
 
+CSD_EDIRECT, CSD_ERING = 8, 9    # a launch wants a form of its kernel attached
 CSD_LOADER_TMA = 0
 CSD_LOADER_LDG = 1
 BC_MODES = {"none": 0, "dirichlet": 1, "neumann": 2, "periodic": 3, "reflecting": 4}
@@ -33,7 +34,19 @@ NVRTC_OPTIONS = (
     "-DNDEBUG",
     "-lineinfo",
     "--ptxas-options=-v",
+    # a module's kernels on several threads: RK4 of a radius-2 operator, twelve
+    # kernels, 7.8 -> 4.0 s on eight cores
+    "--split-compile=0",
 )
+
+# Forms of a kernel that a launch may want beside the kernel itself (csd.h).
+FORM_DIRECT, FORM_RING, FORM_BATCH = 1, 2, 3
+
+
+def form_option(form: int) -> tuple:
+    """NVRTC option that compiles one form of a generated source (0: the
+    kernels themselves)."""
+    return (f"-DCSD_FORM={form}",)
 
 
 class CsdError(RuntimeError):
@@ -122,6 +135,8 @@ def library() -> ctypes.CDLL:
         lib.csd_module_unload.argtypes = [P]
         lib.csd_kernel_get.argtypes = [P, cp, ctypes.POINTER(P)]
         lib.csd_kernel_describe.argtypes = [P, ctypes.POINTER(KernelDesc)]
+        lib.csd_kernel_attach.argtypes = [P, P, ctypes.c_int]
+        lib.csd_kernel_defer.argtypes = [P, ctypes.c_int]
         lib.csd_kernel_ring.argtypes = [P, ctypes.POINTER(P), ctypes.POINTER(ctypes.c_longlong)]
         lib.csd_kernel_resources.argtypes = [P, ctypes.POINTER(ctypes.c_int),
                                              ctypes.POINTER(ctypes.c_int),
@@ -253,38 +268,74 @@ def read_image(path: str, sha256: str | None = None) -> bytes:
 
 class NativeModule:
     """A loaded module (per CUDA context): JIT-compiled from ``src`` with
-    NVRTC, or, given ``image``, a prebuilt cubin of the same source."""
+    NVRTC, or, given ``image``, a prebuilt cubin of the same source.
+
+    A prebuilt cubin holds every form of its kernels.  A JIT-compiled module
+    starts with the kernels themselves; a form is compiled when a launch wants
+    it, as a module of its own (``NativeKernel.need``).  Seconds from source to
+    module on eight cores, all forms at once / the kernels / a form: RK4 of a
+    radius-2 operator FP64 4.8 / 2.7 / 2.2 (direct), 7-point 1.1 / 0.6 / 0.7
+    (direct), 7-point T=4 FP32 4.1 / 2.2 / 1.1 (ring), 2.2 (batch)."""
 
     def __init__(self, src: str, extra_options=(), image: bytes | None = None):
-        lib = library()
-        handle = ctypes.c_void_p()
-        if image is not None:
-            buf = ctypes.create_string_buffer(image, len(image))
-            check(lib.csd_module_load_image(buf, len(image), ctypes.byref(handle)))
-        else:
-            n, hdrs, names = _headers()
-            check(lib.csd_module_load(src.encode(), n, hdrs, names, _options(extra_options),
-                                      default_cache_dir().encode(), ctypes.byref(handle)))
-        self.handle = handle
+        self.src = src if image is None else ""
+        self._options = tuple(extra_options)
+        self._forms: dict[int, ctypes.c_void_p] = {}
+        self._lock = threading.Lock()
         self._kernels: dict[str, NativeKernel] = {}
+        if image is not None:
+            self.handle = ctypes.c_void_p()
+            buf = ctypes.create_string_buffer(image, len(image))
+            check(library().csd_module_load_image(buf, len(image), ctypes.byref(self.handle)))
+        else:
+            self.handle = self._load(0)
+
+    def _load(self, form: int) -> ctypes.c_void_p:
+        handle = ctypes.c_void_p()
+        n, hdrs, names = _headers()
+        check(library().csd_module_load(
+            self.src.encode(), n, hdrs, names, _options(self._options + form_option(form)),
+            default_cache_dir().encode(), ctypes.byref(handle)))
+        return handle
+
+    def form(self, form: int) -> ctypes.c_void_p:
+        """The module of one form of this module's kernels."""
+        with self._lock:
+            m = self._forms.get(form)
+            if m is None:
+                m = self._forms[form] = self._load(form)
+        return m
 
     def kernel(self, name: str) -> "NativeKernel":
         k = self._kernels.get(name)
         if k is None:
+            from cutile.lowering.target_to_cuda import source_forms
+
             handle = ctypes.c_void_p()
             check(library().csd_kernel_get(self.handle, name.encode(), ctypes.byref(handle)))
-            k = NativeKernel(name, handle)
+            k = NativeKernel(name, handle, self, source_forms(self.src, name))
             self._kernels[name] = k
         return k
 
 
 class NativeKernel:
-    def __init__(self, name: str, handle: ctypes.c_void_p):
+    def __init__(self, name: str, handle: ctypes.c_void_p, module: NativeModule | None = None,
+                 forms: tuple = ()):
         self.name = name
         self.handle = handle
+        self._module = module
+        self._missing = set(forms)     # forms of the source that are not attached
         d = KernelDesc()
         check(library().csd_kernel_describe(handle, ctypes.byref(d)))
         self.desc = d.as_dict()
+        for form in self._missing - {FORM_BATCH}:
+            check(library().csd_kernel_defer(handle, form))
+
+    def need(self, form: int) -> None:
+        """Attach a form that the kernel's source holds (compiled on first use)."""
+        if form in self._missing:
+            check(library().csd_kernel_attach(self.handle, self._module.form(form), form))
+            self._missing.discard(form)
 
     def tile_rows(self, shape, halo) -> int:
         """Rows of this kernel's tiles in an array of ``shape``: tiles across
@@ -304,9 +355,11 @@ class NativeKernel:
         six of 32^3 25 and 41, six of 96^3 (6800 tile rows) 92 and 66."""
         ring, below = ctypes.c_void_p(), ctypes.c_longlong()
         check(library().csd_kernel_ring(self.handle, ctypes.byref(ring), ctypes.byref(below)))
-        if not ring.value or (self.desc["ndim"] == 3 and tile_rows >= 16 * below.value):
+        if below.value <= 0 or (self.desc["ndim"] == 3 and tile_rows >= 16 * below.value):
             return self
-        return NativeKernel(self.name, ring)
+        self.need(FORM_RING)
+        check(library().csd_kernel_ring(self.handle, ctypes.byref(ring), ctypes.byref(below)))
+        return NativeKernel(self.name, ring) if ring.value else self
 
     def resources(self) -> dict:
         regs, local, blocks = ctypes.c_int(), ctypes.c_int(), ctypes.c_int()
@@ -495,8 +548,14 @@ def launch(kernel, inputs, outputs, halo, stream=None, *, plans: LaunchPlans | N
     o.bc_value = bc_value
     o.dyn = _pointer(dyn)
     o.red = _pointer(red)
-    check(library().csd_launch(plan.kernel.handle, plan.fin, plan.nin, plan.fout, plan.nout,
-                               plan.opts_ref, stream_handle(stream)))
+    lib, handle = library(), stream_handle(stream)
+    rc = lib.csd_launch(plan.kernel.handle, plan.fin, plan.nin, plan.fout, plan.nout,
+                        plan.opts_ref, handle)
+    if rc in (CSD_EDIRECT, CSD_ERING):
+        plan.kernel.need(FORM_DIRECT if rc == CSD_EDIRECT else FORM_RING)
+        rc = lib.csd_launch(plan.kernel.handle, plan.fin, plan.nin, plan.fout, plan.nout,
+                            plan.opts_ref, handle)
+    check(rc)
 
 
 def grid_size() -> int:
@@ -572,6 +631,7 @@ def launch_batch(kernel: NativeKernel, grids_ptr: int, item_start_ptr: int, ngri
                  total_items: int, stream=None, grid: int = 0, timeout_ns: int = 0,
                  loader: int = 0, grid_index_ptr: int | None = None) -> None:
     lib = library()
+    kernel.need(FORM_BATCH)
     o = LaunchOpts()
     o.grid = grid
     o.loader = loader

@@ -169,6 +169,7 @@ class BatchLaunch:
                                      for g in per_grid))
         if form is not kernel and zchunk == batch_zchunk(kernel):
             zchunk = batch_zchunk(form)      # the usual items of the form that runs
+        form.need(native.FORM_BATCH)     # (not when a capture launches it)
         self.kernel = kernel = form
         gsz = native.grid_size()
         n = len(per_grid)

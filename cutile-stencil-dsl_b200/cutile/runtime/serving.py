@@ -211,6 +211,7 @@ class StencilServer:
                                  f"write one")
             # (which solves will share a batch is not known: the form for small ones)
             kern = prog.kernel("main").batch_form(0)
+            kern.need(native.FORM_BATCH)
             p = (prog, kern, batch_zchunk(kern))
             self._progs[key] = p
         return p

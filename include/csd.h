@@ -34,6 +34,8 @@ extern "C" {
 #define CSD_ETIMEOUT 5    /* a kernel gave up waiting (device error word set) */
 #define CSD_ENODEV 6      /* no CUDA driver or device */
 #define CSD_ENOSYM 7      /* kernel or descriptor missing from a module */
+#define CSD_EDIRECT 8     /* nothing launched: the direct form was deferred, attach it */
+#define CSD_ERING 9       /* nothing launched: the ring form was deferred, attach it */
 
 #define CSD_DTYPE_F32 1
 #define CSD_DTYPE_F64 2
@@ -114,6 +116,23 @@ int csd_module_unload(csd_module* m);
  * and `<name>_desc` descriptor).  Stands in for the generated
  * `<name>_kernel` object (target_to_python.py:34-191). */
 int csd_kernel_get(csd_module* m, const char* name, csd_kernel** out);
+
+/* Forms of a generated kernel beside its own: the direct kernel (rows that are
+ * not aligned), the rings of a register chain (small arrays) and its batched
+ * kernels.  A module holds all of them, or, compiled with -DCSD_FORM=0, none
+ * but the kernel itself, and with -DCSD_FORM=<form> that form alone. */
+#define CSD_FORM_DIRECT 1
+#define CSD_FORM_RING 2
+#define CSD_FORM_BATCH 3
+
+/* Take `form` of the kernel from another module (of the same source). */
+int csd_kernel_attach(csd_kernel* k, csd_module* m, int form);
+
+/* Declare that `form` (CSD_FORM_DIRECT or CSD_FORM_RING) can be attached when
+ * it is wanted: a launch that would take it returns CSD_EDIRECT or CSD_ERING
+ * and has launched nothing, so that it can be repeated after csd_kernel_attach.
+ * While its stream captures, a launch does without the form instead. */
+int csd_kernel_defer(csd_kernel* k, int form);
 
 /* Copy the kernel's compile-time descriptor. */
 int csd_kernel_describe(const csd_kernel* k, csd_kernel_desc* out);
