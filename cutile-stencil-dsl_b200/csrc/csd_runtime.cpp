@@ -354,7 +354,7 @@ struct csd_kernel {
   std::atomic<CUfunction> direct{nullptr};
   csd_kernel_desc direct_desc;
   int direct_blocks_per_sm = 0;
-  unsigned direct_rewrites = 0;   // inputs (bit f) that may be outputs too
+  unsigned direct_rewrites = 0;   // inputs (bit f) that may be outputs too; known at once
   // a register chain's ring form, the faster one on arrays of fewer than
   // ring_below rows of the chain's tiles (csd_launch):
   std::atomic<csd_kernel*> ring{nullptr};
@@ -471,10 +471,6 @@ static bool attach_form(csd_kernel* k, csd_module* m, int form) {
                                                       k->direct_desc.threads, 0) != 0 ||
         k->direct_blocks_per_sm < 1)
       return false;
-    unsigned mask = 0;
-    if (d.cuModuleGetGlobal(&dp, &sz, m->mod, (n + "_direct_rewrites").c_str()) == 0 &&
-        sz == sizeof(mask) && d.cuMemcpyDtoH(&mask, dp, sizeof(mask)) == 0)
-      k->direct_rewrites = mask;
     k->direct = fn;
     return true;
   }
@@ -549,6 +545,10 @@ int csd_kernel_get(csd_module* m, const char* name, csd_kernel** out) {
     }
     if (k->blocks_per_sm[l] < 1) k->blocks_per_sm[l] = 1;
   }
+  unsigned mask = 0;
+  if (d.cuModuleGetGlobal(&dp, &sz, m->mod, (n + "_direct_rewrites").c_str()) == 0 &&
+      sz == sizeof(mask) && d.cuMemcpyDtoH(&mask, dp, sizeof(mask)) == 0)
+    k->direct_rewrites = mask;
   long long below = 0;
   if (d.cuModuleGetGlobal(&dp, &sz, m->mod, (n + "_ring_below").c_str()) == 0 &&
       sz == sizeof(below) && d.cuMemcpyDtoH(&below, dp, sizeof(below)) == 0)

@@ -458,8 +458,6 @@ def _emit_direct(kernel: KernelOp) -> list:
         f"  csd::direct_step<{c}, Body_{name}_direct>(p);",
         "}",
         _descriptor(f"{name}_direct_desc", c, p, 0, min_blocks, 0),
-        *([f'extern "C" __device__ const unsigned {name}_direct_rewrites = {p["REWRITTEN"]};']
-          if p["REWRITTEN"] else []),
         "",
     ]
 
@@ -663,6 +661,9 @@ def emit_cuda(module: ModuleOp, preamble: bool = True) -> str:
             parts.extend(_emit_engine(f"{name}_ring", q))
             parts.append("#endif")
         if direct_plan(kernel)[0]:
+            if p["REWRITTEN"]:      # (read before the direct form is there)
+                parts += ["#if CSD_HAS(0)", f'extern "C" __device__ const unsigned '
+                          f'{name}_direct_rewrites = {p["REWRITTEN"]};', "#endif"]
             parts.append("#if CSD_HAS(1)")
             parts.extend(_emit_direct(kernel))
             parts.append("#endif")

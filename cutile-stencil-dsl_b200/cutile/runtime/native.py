@@ -34,9 +34,6 @@ NVRTC_OPTIONS = (
     "-DNDEBUG",
     "-lineinfo",
     "--ptxas-options=-v",
-    # a module's kernels on several threads: RK4 of a radius-2 operator, twelve
-    # kernels, 7.8 -> 4.0 s on eight cores
-    "--split-compile=0",
 )
 
 # Forms of a kernel that a launch may want beside the kernel itself (csd.h).
@@ -273,9 +270,11 @@ class NativeModule:
     A prebuilt cubin holds every form of its kernels.  A JIT-compiled module
     starts with the kernels themselves; a form is compiled when a launch wants
     it, as a module of its own (``NativeKernel.need``).  Seconds from source to
-    module on eight cores, all forms at once / the kernels / a form: RK4 of a
-    radius-2 operator FP64 4.8 / 2.7 / 2.2 (direct), 7-point 1.1 / 0.6 / 0.7
-    (direct), 7-point T=4 FP32 4.1 / 2.2 / 1.1 (ring), 2.2 (batch)."""
+    module, all forms at once / the kernels / a form: RK4 of a radius-2
+    operator FP64 6.9 / 2.9 / 3.4 (direct), 7-point 1.3 / 0.65 / 0.6 (direct),
+    7-point T=4 FP32 6.8 / 2.8 / 1.3 (ring), 2.7 (batch).  (NVRTC's
+    --split-compile halves these on eight cores, but its kernels take more
+    registers: 27 points FP64 114 for 108, 384^3 242 -> 247 us.)"""
 
     def __init__(self, src: str, extra_options=(), image: bytes | None = None):
         self.src = src if image is None else ""

@@ -67,6 +67,22 @@ def test_a_capture_does_without(fn, ndim, size, form, kw):
     assert form not in kernel._missing and _equal(out, want)
 
 
+@pytest.mark.parametrize("method", ["rk2", "rk4", "ssprk3"])
+def test_every_stage_of_a_step_takes_the_direct_form(method):
+    """Also the stages that rewrite a field they read."""
+    import torch
+
+    from cutile import RKIntegrator, stencil
+
+    r = RKIntegrator(stencil(ndim=2)(D.wave4), method).compile(align_halo=False)
+    mod = r.load_module()
+    u = torch.randn((41, 67), dtype=torch.float64, device="cuda")
+    getattr(mod, f"rk_{method}_step")(u, 0.01)
+    torch.cuda.synchronize()
+    prog = mod.program()
+    assert all(1 not in prog.kernel(k)._missing for k in range(len(prog.table)))
+
+
 def test_launches_of_several_threads_share_the_form():
     import threading
 

@@ -21,6 +21,18 @@ def _lap7(**kw):
     return stencil_compile(stencil(ndim=3, boundary="periodic")(D.lap7), **kw).cuda_source
 
 
+def test_rewritten_fields_are_known_without_the_direct_form():
+    """Whether a launch may take the direct form is decided before it is there."""
+    src = RKIntegrator(stencil(ndim=2)(D.heat2d), "rk4").compile().cuda_source
+    for k, rewrites in enumerate((False, True, True, False)):
+        mark = f"\n__device__ const unsigned* at = &heat2d_rk4_s{k}_direct_rewrites;"
+        if rewrites:
+            native.compile_source(src + mark, native.form_option(0))
+        else:
+            with pytest.raises(native.CsdError):
+                native.compile_source(src + mark, native.form_option(0))
+
+
 @pytest.mark.parametrize("source,names,forms", [
     (lambda: _lap7(temporal_blocking=False), {"lap7": (1,), "lap7_bc": ()},
      [["lap7_tma", "lap7_ldg", "lap7_bc_tma", "lap7_bc_ldg"], ["lap7_direct"], [], []]),
