@@ -395,13 +395,15 @@ def field_of(t, pitched: bool = False) -> Field:
     return f
 
 
-def stream_handle(stream) -> int | None:
+def stream_handle(stream, device: int | None = None) -> int | None:
+    """The CUDA handle of ``stream``, or of the current one (of ``device``,
+    when the caller has asked for the current device already)."""
     import torch
 
     if stream is None:
         raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
         if raw is not None:    # the handle without building a Stream object
-            return raw(torch.cuda.current_device())
+            return raw(torch.cuda.current_device() if device is None else device)
         return torch.cuda.current_stream().cuda_stream
     if isinstance(stream, int):
         return stream
@@ -508,16 +510,16 @@ def launch(kernel, inputs, outputs, halo, stream=None, *, plans: LaunchPlans | N
     ``describe``: a tensor's csd_field where it is not the tensor's own shape
     (what it depends on beside the tensor is part of ``kind``).  Host time of
     one launch call (two fields): 21 -> 10 us, RK4 step 104 -> 48."""
-    plan = key = None
+    plan = key = device = None
     if plans is not None:
         try:
             import torch
 
             # (types stand for the checks that ask for torch tensors, and for an
             # option's own: 1.0 == 1, but is no number of rows)
-            key = (kind, torch.cuda.current_device(), len(inputs), len(scalars),
-                   tuple([(k, type(v), v, tuple(map(type, v)) if type(v) is tuple else None)
-                          for k, v in kw.items()]),
+            device = torch.cuda.current_device()
+            key = (kind, device, len(inputs), len(scalars), tuple(kw.items()),
+                   tuple(map(type, kw.values())), tuple(map(type, kw.get("bc_odd", ()))),
                    tuple([(type(t), t.dtype, t.is_cuda, t.shape, t.stride())
                           for t in (*inputs, *outputs)]))
             plan = plans.by_kind.get(key)
@@ -547,7 +549,7 @@ def launch(kernel, inputs, outputs, halo, stream=None, *, plans: LaunchPlans | N
     o.bc_value = bc_value
     o.dyn = _pointer(dyn)
     o.red = _pointer(red)
-    lib, handle = library(), stream_handle(stream)
+    lib, handle = library(), stream_handle(stream, device)
     rc = lib.csd_launch(plan.kernel.handle, plan.fin, plan.nin, plan.fout, plan.nout,
                         plan.opts_ref, handle)
     if rc in (CSD_EDIRECT, CSD_ERING):

@@ -19,7 +19,7 @@ def launch(monkeypatch):
         return 0
 
     monkeypatch.setattr(native, "library", lambda: SimpleNamespace(csd_launch=csd_launch))
-    monkeypatch.setattr(native, "stream_handle", lambda stream: None)
+    monkeypatch.setattr(native, "stream_handle", lambda stream, device: None)
     monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
     plans = native.LaunchPlans()
     u, v = (torch.zeros(8, 8) for _ in range(2))
