@@ -34,9 +34,8 @@ def reduce(op: int, a, halo, b=None, out=None, stream=None, nblocks: int = DEFAU
         if partials is None:
             partials = torch.empty(nblocks, dtype=torch.float64, device=a.device)
     native.check(lib.csd_reduce(ctypes.byref(fa), ctypes.byref(fb) if fb is not None else None,
-                                h, op, ctypes.c_void_p(partials.data_ptr()), nblocks,
-                                ctypes.c_void_p(out.data_ptr()),
-                                ctypes.c_void_p(native.stream_handle(stream))))
+                                h, op, partials.data_ptr(), nblocks, out.data_ptr(),
+                                native.stream_handle(stream)))
     return out
 
 

@@ -23,7 +23,7 @@ def test_two_streams_share_no_partials(monkeypatch):
 
     class Recorder:
         def csd_reduce(self, *args):
-            seen.append(args[4].value)
+            seen.append(args[4])
             return lib.csd_reduce(*args)
 
         def __getattr__(self, name):
