@@ -557,15 +557,17 @@ def register_chain_plan(radius, dtype_bytes: int, num_inputs: int, T: int, body_
       up to 512^2 (5120), 1.04 to 1.8 at 768^2 (10752); FP32 T = 2 0.7 to 1.05
       up to 4000 x 300 (12000), 1.0 to 2.3 at 1448^2 and 16384 x 64 (16384), T >=
       3 0.4 to 0.9 up to 768^2, 1.02 to 1.5 at 1024^2 (9216);
-    * quotients at radius 1: FP32 0.85 at 512^2, 1.0 to 1.7 at 768^2; FP64 T >= 4
-      0.6 to 1.1 up to 512^2 (4608), 1.2 to 1.6 at 768^2 (10752), T <= 3 0.9 at
-      4096^2; at radius 2 FP64 0.7 to 0.9 at 4096^2: a full division's branches
-      stop the overlap of the stages that the registers live on;
-    * 3-D: FP64 0.8 to 1.0 at 48^3 (96 tile planes), 1.0 to 1.5 at 64^3 (384);
-      FP32 0.65 to 1.0 at 64^3 (192 to 256), 1.0 to 3.0 at 96^3 (384); pointwise and
-      X-only bodies with T = 2 0.5 to 0.9 at 512 x 8 x 512 (4608), 1.0 to 1.3 at
-      256^3 (10240); with quotients 0.3 to 0.5 at 256^3 in FP64, 0.9 to 1.0 in
-      FP32.
+    * quotients at radius 1: FP32 T <= 5 0.85 at 512^2 (2560), 1.0 to 1.7 at 768^2
+      (5376), T = 6 0.94 at 384^2 (1536), 1.1 to 1.4 at 512^2, T = 8 1.0 and more
+      everywhere; FP64 T >= 4 0.6 to 1.1 up to 512^2 (4608), 1.2 to 1.6 at 768^2
+      (10752), T <= 3 0.9 at 4096^2; at radius 2 FP64 0.7 to 0.9 at 4096^2: a
+      full division's branches stop the overlap of the stages that the registers
+      live on;
+    * 3-D: FP64 0.8 to 1.0 at 48^3 (96 tile planes), 1.0 to 1.5 at 64^3 (256 to
+      384), but T = 4 with planes to walk 1.1 and more from 16^3 on; FP32 0.65 to
+      1.0 at 64^3 (192 to 256), 1.0 to 3.0 at 96^3 (384); pointwise and X-only
+      bodies with T = 2 0.5 to 0.9 at 512 x 8 x 512 (4608), 1.0 to 1.3 at 256^3
+      (10240); with quotients 0.3 to 0.5 at 256^3 in FP64, 0.9 to 1.0 in FP32.
 
     In 3-D two rows per thread and sixteen warps while a block of them keeps
     128 registers each, else three rows and eight warps (one row per thread
@@ -574,12 +576,13 @@ def register_chain_plan(radius, dtype_bytes: int, num_inputs: int, T: int, body_
     registers 345)."""
     from cutile.passes.tiling import B200_SMEM_PER_BLOCK
 
-    ndim = len(radius)
+    ndim, fp64 = len(radius), dtype_bytes == 8
     if ndim == 3:
         rz, ry, rx = radius
         vec = 16 // dtype_bytes
         pad = -(-T * rx // vec) * vec
-        below = 8192 if rz == 0 and ry == 0 and T == 2 else 288
+        below = (8192 if rz == 0 and ry == 0 and T == 2 else 0 if rz > 0 and fp64 and T >= 4 else
+                 256 if fp64 else 288)
         for rows, warps, budget in ((2, 16, 84), (3, 8, 210)):
             # 32-bit registers of the T windows: own rows, rows on either side
             words = T * (rows * (2 * rz + 1) + 2 * ry * side_planes) * 4
@@ -597,7 +600,7 @@ def register_chain_plan(radius, dtype_bytes: int, num_inputs: int, T: int, body_
                         "ring_below": below}
         return {}
     rz, rx = (radius[0] if ndim == 2 else 0), radius[-1]
-    r, fp64 = max(rz, rx), dtype_bytes == 8
+    r = max(rz, rx)
     # one 16-byte vector per lane; two in 1-D, where no rows are kept (FP32
     # 2^22: 14.8 us with one, 10.1 with two, 10.2 with four)
     vec = 16 // dtype_bytes * (2 if ndim == 1 else 1)
@@ -613,7 +616,8 @@ def register_chain_plan(radius, dtype_bytes: int, num_inputs: int, T: int, body_
     elif quotients and fp64 and (r > 1 or T <= 3):
         return {}
     elif r <= 1:
-        below = 0 if not quotients else 10240 if fp64 else 4096
+        below = (0 if not quotients else 10240 if fp64 else 4096 if T <= 5 else
+                 2048 if T == 6 else 0)
     elif r == 2 and num_loads <= 9 and not quotients:
         below = (0 if T <= 4 else 2048) if fp64 else (0 if T == 2 else 4096)
     else:
