@@ -726,16 +726,6 @@ def bricked_field(t, shape, brick: int) -> Field:
     return f
 
 
-def launch_fields(kernel: NativeKernel, fin, fout, halo, stream=None, **kw) -> None:
-    """csd_launch on prepared csd_field lists."""
-    lib = library()
-    a = (Field * len(fin))(*fin)
-    b = (Field * max(1, len(fout)))(*fout)
-    o = make_opts(halo, **kw)
-    check(lib.csd_launch(kernel.handle, a, len(fin), b, len(fout), ctypes.byref(o),
-                         ctypes.c_void_p(stream_handle(stream))))
-
-
 CSD_ETIMEOUT = 5
 CSD_ERR_TIMEOUT = 0x7001
 
@@ -759,5 +749,5 @@ def error_word(reset: bool = True) -> int:
 __all__ = ["library", "check", "compile_source", "NativeModule", "NativeKernel", "launch",
            "apply_boundary", "error_word", "error_status", "CSD_ETIMEOUT", "CSD_ERR_TIMEOUT", "CsdError", "field_of", "default_cache_dir",
            "make_opts", "LaunchPlans", "on_stream", "grid_build_rotations", "batch_opts", "grid_size", "grid_build", "launch_batch", "bricked_shape",
-           "to_bricks", "from_bricks", "bricked_field", "launch_fields",
+           "to_bricks", "from_bricks", "bricked_field",
            "GridHead", "plan_items", "NVCC_OPTIONS", "find_nvcc", "aot_compile", "read_image", "CSD_LOADER_TMA", "CSD_LOADER_LDG", "BC_MODES"]
