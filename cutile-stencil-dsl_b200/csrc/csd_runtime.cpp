@@ -658,8 +658,8 @@ static long long split_column(long long nz, long long cnt, int rows, bool shift,
   return n;
 }
 
-// Register chains and direct kernels (engine.cuh ChainCfg, DirectCfg) stage
-// nothing: they have no ring slots.
+// Register chains and direct kernels (engine.cuh ChainCfg, DirectCfg) have no
+// ring slots (a chain's input rows pass through a ring of each thread's own).
 static bool is_register_chain(const csd_kernel_desc& D) { return D.temporal > 1 && D.nslot == 0; }
 static bool is_direct(const csd_kernel_desc& D) {
   return D.temporal == 1 && D.nslot == 0 && D.threads > 0;

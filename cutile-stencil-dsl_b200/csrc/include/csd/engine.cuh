@@ -698,14 +698,15 @@ __device__ __forceinline__ int batch_grid_of(const csd_params& p, int item, int&
 }
 
 // ---------------------------------------------------------------------------
-// Register chains: 1-D and 2-D temporal blocking without shared memory
+// Register chains: 1-D and 2-D temporal blocking in registers
 // ---------------------------------------------------------------------------
 // A work item is one warp's: a strip of TX columns, the warp's 32 x VEC
 // points (VEC neighbouring columns per lane) covering the strip and the
 // columns the T steps consume on either side.  The warp walks the rows of its
 // item with the 2 RZ + 1 newest rows of each of the T fields in registers and
 // reads X neighbours from the neighbouring lanes by shuffles: no barrier and
-// no shared memory stand between the stages.  Stage s reads only rows of
+// no shared memory stand between the stages (the input rows alone pass through
+// it, below).  Stage s reads only rows of
 // field s - 1 that earlier steps finished, so the T stages of a step are
 // independent and hide each other's latency; running them from the last to
 // the first lets the new row of a field take the place of the row that the
@@ -715,7 +716,9 @@ __device__ __forceinline__ int batch_grid_of(const csd_params& p, int item, int&
 // into registers that far ahead measured slower: a step then waits for the
 // youngest of them).  What bounds it is
 // instruction issue: the body's own arithmetic, the shuffles, and the strip's
-// T RX columns and the item's 2 T RZ rows that are computed twice.
+// T RX columns and the item's 2 T RZ rows that are computed twice.  Where those
+// rows outweigh an item's own, or a division's branches keep the stages apart,
+// the ring engine is faster (launcher.register_chain_plan holds the sizes).
 template <typename T_, int NIN_, int NOUT_, int RZ_, int RX_, int NT_, int TEMPORAL_, int LOADER_,
           int VEC_>
 struct ChainCfg {

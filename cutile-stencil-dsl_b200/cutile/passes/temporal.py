@@ -8,8 +8,9 @@ because ``T`` is observable: one ``launch_<name>`` call advances ``T`` steps.
 
 How the steps run is the engine's business: the reference issues ``T``
 launches through scratch buffers; the B200 engine chains the ``T`` steps
-inside one pass over each tile, in shared memory (time skewing), with the
-same result (intermediate steps see zero halos).
+inside one pass over each tile (time skewing), in registers or in
+shared-memory rings (``launcher.register_chain_plan``), with the same result
+(intermediate steps see zero halos).
 """
 
 from __future__ import annotations

@@ -69,7 +69,13 @@ class AotBuild:
 
 @dataclass
 class CompileResult:
-    """Result of compiling a stencil (launcher.py:27-231)."""
+    """Result of compiling a stencil (launcher.py:27-231).
+
+    ``tile_sizes`` and the ``threads``, ``stages``, ``min_blocks`` and ``waves``
+    of ``kernel_hints`` describe the ring engine's plan.  With a
+    ``register_chain`` hint that is the plan of the chain's ring form
+    (``ring_below``); the chain's own tile and block are its kernel's
+    descriptor (``program().kernel().desc``)."""
 
     name: str
     code: str

@@ -73,8 +73,8 @@ typedef struct csd_launch_opts {
                            timeout_ns; the CTA drains its other copies and exits, and
                            csd_error_word then reports CSD_ERR_TIMEOUT.  Nothing faults or
                            hangs: every other CTA finishes normally.  Kernels without a
-                           staging ring (register chains) wait for nothing and ignore it and
-                           timeout_ns. */
+                           staging ring (register chains, which then keep their launches)
+                           wait for nothing and ignore it and timeout_ns. */
 } csd_launch_opts;
 
 /* Library version (major*100 + minor). */
