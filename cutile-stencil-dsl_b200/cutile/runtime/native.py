@@ -511,6 +511,7 @@ def launch(kernel, inputs, outputs, halo, stream=None, *, plans: LaunchPlans | N
     (what it depends on beside the tensor is part of ``kind``).  Host time of
     one launch call (two fields): 21 -> 10 us, RK4 step 104 -> 48."""
     plan = key = device = None
+    fields = (*inputs, *outputs)
     if plans is not None:
         try:
             import torch
@@ -518,16 +519,16 @@ def launch(kernel, inputs, outputs, halo, stream=None, *, plans: LaunchPlans | N
             # (types stand for the checks that ask for torch tensors, and for an
             # option's own: 1.0 == 1, but is no number of rows)
             device = torch.cuda.current_device()
+            odd = kw.get("bc_odd")
             key = (kind, device, len(inputs), len(scalars), tuple(kw.items()),
-                   tuple(map(type, kw.values())), tuple(map(type, kw.get("bc_odd", ()))),
-                   tuple([(type(t), t.dtype, t.is_cuda, t.shape, t.stride())
-                          for t in (*inputs, *outputs)]))
+                   tuple(map(type, kw.values())), odd and tuple(map(type, odd)),
+                   tuple([(type(t), t.dtype, t.is_cuda, t.shape, t.stride()) for t in fields]))
             plan = plans.by_kind.get(key)
         except Exception:  # noqa: BLE001 - not launchable as it is: the checks below say why
             key = None
     if plan is None and check_fields is not None:
         check_fields()
-    ptrs = [t.data_ptr() for t in (*inputs, *outputs)]
+    ptrs = [t.data_ptr() for t in fields]
     if distinct:
         n = len(inputs)
         for p in ptrs[n:]:

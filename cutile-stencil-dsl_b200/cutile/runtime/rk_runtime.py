@@ -64,6 +64,7 @@ class RKProgram:
             ws = {n: tuple(torch.empty_strided(x.size(), x.stride(), dtype=x.dtype,
                                                device=x.device).zero_() for x in state)
                   for n in sorted(names)}
+            ws["dt"] = torch.empty(1, dtype=torch.float64, device=state[0].device)
             self._work[key] = ws
         return ws
 
@@ -95,25 +96,28 @@ class RKProgram:
         m = self.spec["state_fields"]
         if len(fields) + len(aux) != self.spec["fields"]:
             raise TypeError(f"the operator reads {self.spec['fields']} fields")
+        rest = fields[m:] + tuple(aux)
+        if stream is None:
+            return self._step(fields[:m], rest, dt, stream, scalars)
         # dt, the workspace's first zeros and the final copy are part of the
-        # step: in its stream's order, with a dt scalar of the step's own
+        # step, in its stream's order; dt is a scalar of the state's workspace, so
+        # that steps of several states overlap
         with native.on_stream(stream):
-            self._step(fields[:m], tuple(fields[m:]) + tuple(aux), dt, stream, scalars)
+            self._step(fields[:m], rest, dt, stream, scalars)
 
     def _step(self, state: tuple, rest: tuple, dt, stream, scalars: dict | None) -> None:
         import torch
 
-        dyn = dt if isinstance(dt, torch.Tensor) else torch.full(
-            (1,), float(dt), dtype=torch.float64, device=state[0].device)
         bufs = dict(self.workspace(state))
         bufs["u"] = state
+        dyn = dt if isinstance(dt, torch.Tensor) else bufs["dt"].fill_(float(dt))
         sv = self._scalars(scalars)
-        halo = self.spec["halo"]
+        halo, odd = self.spec["halo"], tuple(self.bc_odd)
         for k in range(len(self.table)):
             inputs, outputs = self.stage_io(k, bufs, rest)
             native.launch(lambda: self.kernel(k), inputs, outputs, halo, stream,  # noqa: B023
-                          plans=self._plans, kind=k, scalars=sv, dyn=dyn,
-                          bc_odd=tuple(self.bc_odd), bc_value=self.bc_value)
+                          plans=self._plans, kind=k, scalars=sv, dyn=dyn, bc_odd=odd,
+                          bc_value=self.bc_value)
         last_out = self.table[-1][7]
         if last_out != "u":
             inner = tuple(slice(h, s - h) for h, s in zip(halo, state[0].shape))
