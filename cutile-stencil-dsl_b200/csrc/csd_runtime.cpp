@@ -355,8 +355,8 @@ struct csd_kernel {
   csd_kernel_desc direct_desc;
   int direct_blocks_per_sm = 0;
   unsigned direct_rewrites = 0;   // inputs (bit f) that may be outputs too; known at once
-  // a register chain's ring form, the faster one on arrays of fewer than
-  // ring_below rows of the chain's tiles (csd_launch):
+  // a register chain's ring form, the faster one on arrays below ring_below
+  // (chain_size):
   std::atomic<csd_kernel*> ring{nullptr};
   long long ring_below = 0;
   // the kernels that batches launch (their own in register chains):
@@ -1002,6 +1002,14 @@ static int build_grid(csd_kernel* k, const csd_field* in, int n_in, const csd_fi
   return CSD_OK;
 }
 
+// What the rings of a chain would work on in a grid: rows of 128 columns, or in
+// 3-D planes of the chain's tiles.
+static long long chain_size(const csd_grid& g) {
+  const long long across =
+      g.ndim == 3 ? (long long)g.tiles[0] * g.tiles[1] : (g.interior[2] + 127) / 128;
+  return across * g.interior[0];
+}
+
 int csd_launch(csd_kernel* k, const csd_field* in, int n_in, const csd_field* out, int n_out,
                const csd_launch_opts* opts, void* stream) {
   if (!k) return fail(CSD_EINVAL, "null kernel");
@@ -1032,7 +1040,7 @@ int csd_launch(csd_kernel* k, const csd_field* in, int n_in, const csd_field* ou
   // 25 / 33), so a quarter of the size decides there.
   const long long limit = loader == CSD_LOADER_TMA ? k->ring_below : k->ring_below / 4;
   if (limit > 0 && (o.loader < 0 || o.loader > 1) && o.zchunk <= 0 && o.withhold_chunk <= 0 &&
-      (long long)p.g.tiles[0] * p.g.tiles[1] * p.g.interior[0] < limit) {
+      chain_size(p.g) < limit) {
     if (k->ring) {
       k = k->ring;
       rc = build_grid(k, in, n_in, out, n_out, o, st, false, stream, &p.g, &loader);

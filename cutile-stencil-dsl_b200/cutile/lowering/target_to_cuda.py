@@ -532,7 +532,7 @@ def engine_params(kernel: KernelOp, ring: bool = False) -> dict:
         "OCCUPANCY": int(hints.get("occupancy", 0)),   # a caller's blocks per SM (0: none)
         # points per lane of a register chain (0: the ring engine)
         "CHAIN": int(hints.get("register_chain", 0)),
-        # rows of its tiles from which the chain is the faster form (0: always)
+        # size from which the chain is the faster form (0: always)
         "RING_BELOW": int(hints.get("ring_below", 0)),
         "VEC": int(hints.get("register_chain", 0)
                    or hints.get("vec", 4 if dtype in ("float32", "fp32") else 2)),

@@ -550,30 +550,33 @@ def register_chain_plan(radius, dtype_bytes: int, num_inputs: int, T: int, body_
     329 -> 212, T=4 982 -> 487; FP32 T=2 186 -> 148, T=4 559 -> 423.
 
     An item computes T rz rows more than it stores on either side, so a chain
-    has to have enough rows of its tiles (tiles across X and Y, times the rows
-    or planes of each: ``ring_below`` counts these) for long items; the rings
-    share such rows between the threads of a block.  Ratio rings / registers:
+    has to have enough rows for long items; the rings share such rows between
+    the threads of a block, but work on tiles 128 columns wide, however narrow
+    the array.  ``ring_below`` counts what the rings would work on: rows of
+    128 columns, in 3-D planes of the chain's tiles.  Ratio rings / registers,
+    the sizes in brackets:
     * radius 1 without quotients (5 and 9 points, 1-D, T = 2 to 8): 1.0 and
       more from 64^2 on, so always registers;
-    * 9-point stars of radius 2: FP64 T <= 4 1.0 and more everywhere, T = 6 0.92
-      at 256^2 (1280 tile rows) and 1.2 at 384^2 (2688); FP32 T = 2 1.05 and
-      more, T = 3 to 6 0.7 to 0.9 from 256^2 to 512^2 (2560), 1.1 to 1.6 at
-      768^2 (5376), 1.8 to 2.5 at 4096 x 20 (4096);
-    * denser footprints, radius 3, FP32 quotients at radius 2: FP64 0.3 to 1.1
-      up to 512^2 (5120), 1.04 to 1.8 at 768^2 (10752); FP32 T = 2 0.7 to 1.05
-      up to 4000 x 300 (12000), 1.0 to 2.3 at 1448^2 and 16384 x 64 (16384), T >=
-      3 0.4 to 0.9 up to 768^2, 1.02 to 1.5 at 1024^2 (9216);
-    * quotients at radius 1: FP32 T <= 5 0.85 at 512^2 (2560), 1.0 to 1.7 at 768^2
-      (5376), T = 6 0.94 at 384^2 (1536), 1.1 to 1.4 at 512^2, T = 8 1.0 and more
-      everywhere; FP64 T >= 4 0.6 to 1.1 up to 512^2 (4608), 1.2 to 1.6 at 768^2
-      (10752), T <= 3 0.9 at 4096^2; at radius 2 FP64 0.7 to 0.9 at 4096^2: a
-      full division's branches stop the overlap of the stages that the registers
-      live on;
-    * 3-D: FP64 0.8 to 1.0 at 48^3 (96 tile planes), 1.0 to 1.5 at 64^3 (256 to
-      384), but T = 4 with planes to walk 1.1 and more from 16^3 on; FP32 0.65 to
-      1.0 at 64^3 (192 to 256), 1.0 to 3.0 at 96^3 (384); pointwise and X-only
-      bodies with T = 2 0.5 to 0.9 at 512 x 8 x 512 (4608), 1.0 to 1.3 at 256^3
-      (10240); with quotients 0.3 to 0.5 at 256^3 in FP64, 0.9 to 1.0 in FP32.
+    * 9-point stars of radius 2: FP64 T <= 5 and FP32 T = 2 1.0 and more
+      everywhere, FP64 T = 6 0.85 at 256^2 [512] and 1.2 at 384^2 [1152]; FP32 T =
+      3 to 5 0.7 to 0.96 from 256^2 to 512^2 [2048], 1.1 to 2.5 at 768^2 [4608]
+      and 4096 x 20 [4096]; T = 6 0.7 at 384^2, 1.1 at 512^2;
+    * denser footprints, radius 3, FP32 quotients at radius 2: FP64 0.3 to 1.4
+      up to 512^2 [2048], 1.04 to 3.5 at 768^2 and 4096 x 20; FP32 T = 2 0.6 to
+      1.05 up to 4000 x 300 [12000], 1.0 to 2.3 at 1448^2 [17376] and 16384 x 64
+      [16384]; T >= 3 0.3 to 1.08 at 768^2, 1.02 to 2.1 at 1024^2 [8192] and
+      8 x 100000 [6256];
+    * quotients at radius 1: FP32 T = 3 to 5 0.85 to 0.9 at 512^2, 1.1 to 1.7 at
+      768^2, T = 2 0.92 (1 us) and more everywhere, T >= 6 0.85 to 1.0 at 384^2,
+      1.1 to 1.5 at 512^2; FP64 T = 4 and 5 0.6 to 1.04 up to 512^2, 1.2 to 2.6 at
+      768^2 and 4096 x 20, T >= 6 1.1 and more from 512^2, T <= 3 0.9 at 4096^2; at
+      radius 2 FP64 0.7 to 0.9 at 4096^2: a full division's branches stop the
+      overlap of the stages that the registers live on;
+    * 3-D: FP64 0.8 to 1.0 at 48^3 [96], 1.0 to 1.5 at 64^3 [256 to 384], but T =
+      4 with planes to walk 1.1 and more from 16^3 on; FP32 0.65 to 1.0 at 64^3
+      [192 to 256], 1.0 to 3.0 at 96^3 [384]; pointwise and X-only bodies with T =
+      2 0.5 to 0.9 at 512 x 8 x 512 [4608], 1.0 to 1.3 at 256^3 [10240]; with
+      quotients 0.3 to 0.5 at 256^3 in FP64, 0.9 to 1.0 in FP32.
 
     In 3-D two rows per thread and sixteen warps while a block of them keeps
     128 registers each, else three rows and eight warps (one row per thread
@@ -618,16 +621,16 @@ def register_chain_plan(radius, dtype_bytes: int, num_inputs: int, T: int, body_
     if window > 192 or T * (2 * rz + 1) * body_ops > 2000:
         return {}
     if ndim == 1:
-        below = 2048 if quotients and fp64 and T <= 3 else 0
+        below = 1024 if quotients and fp64 and T <= 3 else 0
     elif quotients and fp64 and (r > 1 or T <= 3):
         return {}
     elif r <= 1:
-        below = (0 if not quotients else 10240 if fp64 else 4096 if T <= 5 else
-                 2048 if T == 6 else 0)
+        below = 0 if not quotients else ((4096 if T <= 5 else 2048) if fp64 else
+                                         0 if T == 2 else 4096 if T <= 5 else 1536)
     elif r == 2 and num_loads <= 9 and not quotients:
-        below = (0 if T <= 4 else 2048) if fp64 else (0 if T == 2 else 4096)
+        below = (0 if T <= 5 else 768) if fp64 else 0 if T == 2 else 4096 if T <= 5 else 2048
     else:
-        below = 10240 if fp64 else 16384 if T == 2 else 8192
+        below = 4096 if fp64 else 16384 if T == 2 else 6144
     # the strip's stored columns: at least half of the 32 lanes' points
     pad = -(-T * rx // vec) * vec
     if 2 * (32 * vec - pad - T * rx) < 32 * vec:

@@ -336,25 +336,24 @@ class NativeKernel:
             check(library().csd_kernel_attach(self.handle, self._module.form(form), form))
             self._missing.discard(form)
 
-    def tile_rows(self, shape, halo) -> int:
-        """Rows of this kernel's tiles in an array of ``shape``: tiles across
-        its interior, times the rows (3-D: planes) of each."""
+    def chain_size(self, shape, halo) -> int:
+        """Size of an array of ``shape`` as a chain's ``ring_below`` counts it:
+        rows of 128 columns, in 3-D planes of the kernel's tiles."""
         n = [s - 2 * h for s, h in zip(shape, halo)]
-        across = -(-n[-1] // self.desc["tile_x"])
         if len(n) == 3:
-            across *= -(-n[1] // self.desc["tile_y"])
-        return across * (n[0] if len(n) > 1 else 1)
+            return -(-n[2] // self.desc["tile_x"]) * -(-n[1] // self.desc["tile_y"]) * n[0]
+        return -(-n[-1] // 128) * (n[0] if len(n) > 1 else 1)
 
-    def batch_form(self, tile_rows: int) -> "NativeKernel":
-        """The form of this kernel for a batch of ``tile_rows`` in all: the
-        ring form of a register chain that has one, but for 3-D batches of
-        sixteen times the rows from which a launch alone takes the chain.
+    def batch_form(self, size: int) -> "NativeKernel":
+        """The form of this kernel for a batch of ``size`` (``chain_size``) in
+        all: the ring form of a register chain that has one, but for 3-D batches
+        of sixteen times the size from which a launch alone takes the chain.
         A batch's items are 16 rows, which favours the rings: 25 points FP64
         T=3, 16 grids of 1026^2, rings 426 us, registers 624; 7 points FP64 T=2,
-        six of 32^3 25 and 41, six of 96^3 (6800 tile rows) 92 and 66."""
+        six of 32^3 25 and 41, six of 96^3 (size 6800) 92 and 66."""
         ring, below = ctypes.c_void_p(), ctypes.c_longlong()
         check(library().csd_kernel_ring(self.handle, ctypes.byref(ring), ctypes.byref(below)))
-        if below.value <= 0 or (self.desc["ndim"] == 3 and tile_rows >= 16 * below.value):
+        if below.value <= 0 or (self.desc["ndim"] == 3 and size >= 16 * below.value):
             return self
         self.need(FORM_RING)
         check(library().csd_kernel_ring(self.handle, ctypes.byref(ring), ctypes.byref(below)))

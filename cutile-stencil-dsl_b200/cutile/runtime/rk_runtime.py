@@ -169,7 +169,7 @@ class BatchLaunch:
                  bc_value: float = 0.0):
         import torch
 
-        form = kernel.batch_form(sum(kernel.tile_rows(g["inputs"][0].shape, halo)
+        form = kernel.batch_form(sum(kernel.chain_size(g["inputs"][0].shape, halo)
                                      for g in per_grid))
         if form is not kernel and zchunk == batch_zchunk(kernel):
             zchunk = batch_zchunk(form)      # the usual items of the form that runs

@@ -144,10 +144,10 @@ int csd_kernel_resources(csd_kernel* k, int* regs, int* local_bytes, int* blocks
 
 /* The ring form of a register chain (`<name>_ring`, the same steps staged in
  * shared memory), or null: csd_launch takes it for arrays of fewer than
- * `*below` rows of the chain's tiles (tiles across X and Y, times the rows of
- * dim 0; a quarter where rows are not aligned), unless opts ask for items
- * (`zchunk`) or a copy path.  A batch keeps the kernel that it is given:
- * callers look the ring form up here. */
+ * `*below` rows of 128 columns (3-D: planes of the chain's tiles; a quarter
+ * where rows are not aligned), unless opts ask for items (`zchunk`) or a copy
+ * path.  A batch keeps the kernel that it is given: callers look the ring form
+ * up here. */
 int csd_kernel_ring(const csd_kernel* k, csd_kernel** ring, long long* below);
 
 /* One stencil pass: read `in[0..n_in)`, write the interior of

@@ -33,8 +33,8 @@ def ratio(u, dx, i, j):
     (star2, 2, "float32", 2, 16384), (star2, 2, "float64", 2, None),
     (star2_half, 2, "float64", 2, 0),            # a quotient by 4 is a product
     (ratio, 2, "float64", 2, 0),                 # a quotient of scalars is no field's
-    (mean9, 2, "float32", 4, 4096), (mean9, 2, "float32", 6, 2048), (mean9, 2, "float32", 8, 0),
-    (mean9, 2, "float64", 5, 10240),
+    (mean9, 2, "float32", 4, 4096), (mean9, 2, "float32", 2, 0), (mean9, 2, "float32", 6, 1536),
+    (mean9, 2, "float64", 5, 4096), (mean9, 2, "float64", 6, 2048),
     (mean9, 2, "float64", 2, None),
     (D.lap7, 3, "float64", 2, 256), (D.lap7, 3, "float64", 4, 0), (D.lap7, 3, "float32", 4, 288),
     (D.lap3d, 3, "float64", 2, None), (D.lap3d, 3, "float32", 3, None)])

@@ -23,8 +23,9 @@ def _compiled(fn, ndim, dtype, T, **kw):
     (star2, 2, "float32", 2), (D.wave4, 2, "float32", 4)])
 @pytest.mark.parametrize("align_halo", [True, False])
 def test_either_side_of_the_limit(fn, ndim, dtype, T, align_halo):
-    """A row less than the limit and the limit itself over two tiles, the last
-    one ragged, a dimension; asked for by loader or items a launch keeps the chain."""
+    """A row less than the limit and the limit itself (2-D: three ragged tiles of
+    128 columns; 3-D: two by two of the chain's), odd rows too; asked for by
+    loader or items a launch keeps the chain."""
     import torch
 
     r = _compiled(fn, ndim, dtype, T, align_halo=align_halo)
@@ -33,11 +34,12 @@ def test_either_side_of_the_limit(fn, ndim, dtype, T, align_halo):
     d, below = kern.desc, r.kernel_hints["ring_below"]
     ring = kern.batch_form(below - 1)
     assert ring.desc["nslot"] > 0 and d["nslot"] == 0
-    across = (d["tile_x"] + 9,) if ndim == 2 else (d["tile_y"] + 1, d["tile_x"] + 9)
+    across = (2 * 128 + 9,) if ndim == 2 else (d["tile_y"] + 1, d["tile_x"] + 9)
+    limit = -(-below // (3 if ndim == 2 else 4))
     rng = np.random.default_rng(T)
-    for rows in (below // 2 ** (ndim - 1) - 1, below // 2 ** (ndim - 1)):
+    for rows in (limit - 1, limit):
         shape = tuple(s + 2 * h for s, h in zip((rows,) + across, r.halo_widths))
-        assert (kern.tile_rows(shape, r.halo_widths) < below) == (rows < below // 2 ** (ndim - 1))
+        assert (kern.chain_size(shape, r.halo_widths) < below) == (rows < limit)
         u = rng.standard_normal(shape).astype(dtype)
         want = O.temporal_launch(u, np.full(shape, np.nan, dtype=dtype), fn, ndim, r.halo_widths, T)
         t = torch.from_numpy(u).cuda()
@@ -50,7 +52,7 @@ def test_either_side_of_the_limit(fn, ndim, dtype, T, align_halo):
 @pytest.mark.parametrize("fn,ndim,dtype,T,sides", [
     (D.lap7, 3, "float64", 2, (9, 33, 40)), (D.lap7, 3, "float32", 2, (300, 290, 280)),
     (star2, 2, "float32", 2, (65, 130)), (D.heat2d, 2, "float64", 5, (33, 258, 120))])
-def test_batches_take_the_form_for_their_rows(fn, ndim, dtype, T, sides):
+def test_batches_take_the_form_for_their_size(fn, ndim, dtype, T, sides):
     import torch
 
     from cutile.runtime.rk_runtime import BatchLaunch, batch_zchunk, pack_grids
@@ -67,9 +69,9 @@ def test_batches_take_the_form_for_their_rows(fn, ndim, dtype, T, sides):
         alone.append(torch.zeros(src.shape, dtype=src.dtype, device="cuda"))
         prog.launch([src.contiguous()], [alone[-1]], loader=1)
     batch = BatchLaunch(kern, per, r.halo_widths, zchunk=batch_zchunk(kern))
-    rows = sum(kern.tile_rows(s, r.halo_widths) for s in shapes)
+    size = sum(kern.chain_size(s, r.halo_widths) for s in shapes)
     below = r.kernel_hints["ring_below"]
-    assert (batch.kernel.desc["nslot"] > 0) == (below > 0 and (ndim < 3 or rows < 16 * below))
+    assert (batch.kernel.desc["nslot"] > 0) == (below > 0 and (ndim < 3 or size < 16 * below))
     batch.launch()
     torch.cuda.synchronize()
     for (_, dst), want in zip(grids, alone):
